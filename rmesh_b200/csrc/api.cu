@@ -117,10 +117,11 @@ struct RmeshCtx {
   // per (tet, view) item, at tet * n_views + view: tiles touched, projections,
   // tile-kernel record; compacted sort keys and values (item indices)
   DevBuf vis_key, vis_val, vis_cnt, vis_proj, vis_view, vis_key_alt, vis_val_alt, group_off;
-  DevBuf vis_color, vis_dcolor;  // SH colours per entry and their gradients
+  DevBuf vis_color;              // SH colours per entry
+  DevBuf mom;                    // adjoint moments per entry (error statistics: per tet)
   DevBuf pair_key, pair_val, pair_key_alt, pair_val_alt, ranges;
   DevBuf rgba, aux, dl, gt, out_a, out_b, out_c, out_d;
-  DevBuf spans_fwd, spans_adj;  // per sorted pair: pixel spans of its tile rows (forward / adjoint rule)
+  DevBuf spans_fwd, spans_adj;  // per sorted pair: span words of its tile rows (forward / adjoint rule)
   DevBuf tile_order, order_hist;  // longest-first tile order of the run; bucket counts and cursors
   DevBuf tickets;                 // persistent tile-queue heads, one per launch of a run
   DevBuf err_in, err_out;  // per-pixel error inputs, per-tet error statistics
@@ -315,7 +316,6 @@ struct TileConf {
 constexpr int kMaxTileGroups = 8;
 
 int conf_threads(TileConf t) { return (t.wide ? 2 : 1) * (((t.ts * t.ts + 31) / 32) * 32); }
-int conf_minb(TileConf t) { return (t.wide ? 1 : 2) * (t.ts == 16 ? 1 : (t.ts == 12 ? 2 : 4)); }
 bool conf_from(int ts, int threads, TileConf* out) {
   if (ts != 8 && ts != 12 && ts != 16) return false;
   TileConf t{ts, 0};
@@ -417,15 +417,14 @@ int ensure_run_buffers(RmeshCtx* c, int n_views, uint64_t total_pixels, uint32_t
   CKR(ensure_buf(c, c->vis_view, items * sizeof(TetView)));
   if (c->sh_degree >= 0) {
     CKR(ensure_buf(c, c->vis_color, items * 16));
-    CKR(ensure_buf(c, c->vis_dcolor, items * 16));
   }
   if (c->cap_pairs == 0) c->cap_pairs = std::max<uint64_t>(8 * items, 1u << 16);
   CKR(ensure_buf(c, c->pair_key, c->cap_pairs * 4));
   CKR(ensure_buf(c, c->pair_val, c->cap_pairs * 4));
   CKR(ensure_buf(c, c->pair_key_alt, c->cap_pairs * 4));
   CKR(ensure_buf(c, c->pair_val_alt, c->cap_pairs * 4));
-  CKR(ensure_buf(c, c->spans_fwd, c->cap_pairs * kSpanRec));
-  CKR(ensure_buf(c, c->spans_adj, c->cap_pairs * kSpanRec));
+  CKR(ensure_buf(c, c->spans_fwd, c->cap_pairs * 4 * kSpanWords));
+  CKR(ensure_buf(c, c->spans_adj, c->cap_pairs * 4 * kSpanWords));
   const uint64_t sort_items = std::max<uint64_t>(std::max<uint64_t>(items, c->cap_pairs), 4ull * c->M);
   CKR(ensure_buf(c, c->sort_status, ((sort_items + kSortPart - 1) / kSortPart + 1) * 256 * 8));
   CKR(ensure_buf(c, c->scan_status, ((items + 255) / 256 + 2) * 8));
@@ -625,8 +624,9 @@ int run_bin(RmeshCtx* c, const ViewParams* views_dev, int n_views, uint32_t tota
     sa.n_ptr = &cnt->n_pairs;
     sa.cap = c->cap_pairs;
     sa.vis_view = c->vis_view.as<TetView>();
-    sa.spans_fwd = c->spans_fwd.as<uint8_t>();
-    sa.spans_adj = c->spans_adj.as<uint8_t>();
+    sa.spans_fwd = c->spans_fwd.as<uint32_t>();
+    sa.spans_adj = c->spans_adj.as<uint32_t>();
+    sa.stride = c->cap_pairs;
     const int sblocks = (int)std::min<uint64_t>((c->cap_pairs + 255) / 256, (uint64_t)c->num_sms * 8);
     pair_spans_kernel<<<std::max(1, sblocks), 256, 0, c->stream>>>(sa);
     CKL();
@@ -650,28 +650,29 @@ int run_bin(RmeshCtx* c, const ViewParams* views_dev, int n_views, uint32_t tota
   return RMESH_OK;
 }
 
-template <int TS, int MODE, bool AUX, bool WIDE>
+template <int TS, int SR, int MODE, bool AUX>
 int launch_tile_t(RmeshCtx* c, TileArgs& ta, uint32_t n_tiles, bool persistent) {
-  constexpr int NT = TileCfg<TS, AUX, WIDE>::NT;
-  constexpr size_t smem = sizeof(TileSmem<TS, AUX, WIDE>);
+  constexpr int NT = 32 * kStripWarps;
+  constexpr size_t smem = kStripWarps * sizeof(StripSmem<TS, SR, AUX>);
   static PerDeviceOnce attrs;  // per instantiation and device
   CK(attrs.run([]() -> cudaError_t {
-    cudaError_t e = cudaFuncSetAttribute(tile_kernel<TS, MODE, AUX, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(strip_kernel<TS, SR, MODE, AUX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     // the whole unified L1 as shared memory: resident CTAs are limited by it
-    return cudaFuncSetAttribute(tile_kernel<TS, MODE, AUX, WIDE>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    return cudaFuncSetAttribute(strip_kernel<TS, SR, MODE, AUX>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                 (int)cudaSharedmemCarveoutMaxShared);
   }));
-  unsigned grid = n_tiles;
+  const uint64_t units = (uint64_t)n_tiles * StripCfg<TS, SR>::S;
+  if (units >= (1ull << 31)) return fail(c, RMESH_ERR_INVALID_ARG, "too many tiles in one launch");
+  unsigned grid = (unsigned)((units + kStripWarps - 1) / kStripWarps);
   if (persistent) {
     int occ = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, tile_kernel<TS, MODE, AUX, WIDE>, NT, smem);
-    grid = (unsigned)std::max(1, occ) * (unsigned)c->num_sms;
-    grid = std::min<unsigned>(grid, std::max<uint32_t>(n_tiles, 1));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, strip_kernel<TS, SR, MODE, AUX>, NT, smem);
+    grid = std::min<unsigned>((unsigned)std::max(1, occ) * (unsigned)c->num_sms, std::max(1u, grid));
   }
   ta.persistent = persistent ? 1 : 0;
   if (grid == 0) return RMESH_OK;
-  tile_kernel<TS, MODE, AUX, WIDE><<<grid, NT, smem, c->stream>>>(ta);
+  strip_kernel<TS, SR, MODE, AUX><<<grid, NT, smem, c->stream>>>(ta);
   CKL();
   return RMESH_OK;
 }
@@ -681,12 +682,12 @@ template <int MODE, bool AUX>
 int launch_tile_m(RmeshCtx* c, TileArgs& ta, uint32_t n_tiles, bool persistent, TileConf tc) {
   const int key = tc.ts * 2 + (tc.wide ? 1 : 0);
   switch (key) {
-    case 16: return launch_tile_t<8, MODE, AUX, false>(c, ta, n_tiles, persistent);
-    case 17: return launch_tile_t<8, MODE, AUX, true>(c, ta, n_tiles, persistent);
-    case 24: return launch_tile_t<12, MODE, AUX, false>(c, ta, n_tiles, persistent);
-    case 25: return launch_tile_t<12, MODE, AUX, true>(c, ta, n_tiles, persistent);
-    case 32: return launch_tile_t<16, MODE, AUX, false>(c, ta, n_tiles, persistent);
-    case 33: return launch_tile_t<16, MODE, AUX, true>(c, ta, n_tiles, persistent);
+    case 16: return launch_tile_t<8, 4, MODE, AUX>(c, ta, n_tiles, persistent);
+    case 17: return launch_tile_t<8, 2, MODE, AUX>(c, ta, n_tiles, persistent);
+    case 24: return launch_tile_t<12, 4, MODE, AUX>(c, ta, n_tiles, persistent);
+    case 25: return launch_tile_t<12, 2, MODE, AUX>(c, ta, n_tiles, persistent);
+    case 32: return launch_tile_t<16, 4, MODE, AUX>(c, ta, n_tiles, persistent);
+    case 33: return launch_tile_t<16, 2, MODE, AUX>(c, ta, n_tiles, persistent);
     default: return fail(c, RMESH_ERR_INVALID_ARG, "tile size must be 8, 12 or 16");
   }
 }
@@ -718,26 +719,42 @@ TileArgs base_tile_args(RmeshCtx* c, const ViewParams* views_dev, int n_views, u
   ta.vis_view = c->vis_view.as<TetView>();
   ta.rec = c->rec.as<TetRec>();
   ta.color4 = c->color4.as<float4>();
-  ta.color_view_stride = 0;
-  ta.grad_slot = c->grad_slot.as<float>();
-  if (c->sh_degree >= 0) {
-    ta.vis_color = c->vis_color.as<float4>();
-    ta.vis_dcolor = c->vis_dcolor.as<float4>();
-  }
+  ta.mom = c->mom.as<float>();
+  if (c->sh_degree >= 0) ta.vis_color = c->vis_color.as<float4>();
   ta.counters = cnt;
   ta.hp = c->hp_d.as<AdamParams>();
-  ta.spans_fwd = c->spans_fwd.as<uint8_t>();
-  ta.spans_adj = c->spans_adj.as<uint8_t>();
+  ta.spans_fwd = c->spans_fwd.as<uint32_t>();
+  ta.spans_adj = c->spans_adj.as<uint32_t>();
+  ta.span_stride = c->cap_pairs;
   ta.tile_order = c->tile_order.as<uint32_t>();
   ta.tile_lo = 0;
   ta.ticket = c->tickets.as<uint32_t>();
   return ta;
 }
 
-// SH colours: clears the per-entry colour gradients before an adjoint launch
-int clear_dcolor(RmeshCtx* c, int n_views) {
-  if (c->sh_degree < 0) return RMESH_OK;
-  CK(cudaMemsetAsync(c->vis_dcolor.p, 0, (size_t)n_views * c->M * 16, c->stream));
+// moments of every entry (ensured before a capture, cleared before an adjoint launch)
+int ensure_moments(RmeshCtx* c, int n_views) {
+  return ensure_buf(c, c->mom, (size_t)n_views * c->M * kMom * 4);
+}
+int clear_moments(RmeshCtx* c, int n_views) {
+  CK(cudaMemsetAsync(c->mom.p, 0, (size_t)n_views * c->M * kMom * 4, c->stream));
+  return RMESH_OK;
+}
+
+// the tets' gradients from an adjoint launch's moments
+int run_grad_finalize(RmeshCtx* c, const ViewParams* views_dev, int n_views, bool capturing) {
+  StageScope sc(c, kStComposite, capturing);
+  GradFinalizeArgs ga;
+  ga.M = (int)c->M;
+  ga.n_views = n_views;
+  ga.views = views_dev;
+  ga.rec = c->rec.as<TetRec>();
+  ga.vis_cnt = c->vis_cnt.as<uint32_t>();
+  ga.mom = c->mom.as<float>();
+  ga.grad_slot = c->grad_slot.as<float>();
+  ga.sh = c->sh_degree >= 0 ? 1 : 0;
+  grad_finalize_kernel<<<(unsigned)((c->M + 127) / 128), 128, 0, c->stream>>>(ga);
+  CKL();
   return RMESH_OK;
 }
 
@@ -752,7 +769,7 @@ int run_sh_backward(RmeshCtx* c, const ViewParams* views_dev, int n_views, bool 
   sa.rec = c->rec.as<TetRec>();
   sa.sh = c->sh.as<float>();
   sa.vis_cnt = c->vis_cnt.as<uint32_t>();
-  sa.vis_dcolor = c->vis_dcolor.as<float4>();
+  sa.mom = c->mom.as<float>();
   sa.d_sh = sh_grad(c);
   sa.grad_slot = c->grad_slot.as<float>();
   const unsigned blocks = (unsigned)((c->M + 127) / 128);
@@ -857,6 +874,7 @@ int train_views(RmeshCtx* c, const RmeshCamera* cams, int n_views, const float* 
   const bool direct_gt = is_device_ptr(gt);
   for (int attempt = 0; attempt < 4; ++attempt) {
     CKR(ensure_run_buffers(c, run_views, total_pix, plain ? max_tiles : total_tiles));
+    CKR(ensure_moments(c, run_views));
     if (!direct_gt) CKR(ensure_buf(c, c->gt, total_pix * 12));
     AdamParams& hp = *c->hp_h;
     hp.step = c->step + 1;
@@ -887,24 +905,26 @@ int train_views(RmeshCtx* c, const RmeshCamera* cams, int n_views, const float* 
           const TileConf tc = pl.conf[pl.order[i]];
           const std::vector<TileGroup> one{TileGroup{tc, 0u, vt}};
           CKR(run_bin(c, vd + i, 1, vt, cnt + i, capturing, one));
-          CKR(clear_dcolor(c, 1));
+          CKR(clear_moments(c, 1));
           {
             StageScope sc(c, kStComposite, capturing);
             TileArgs ta = base_tile_args(c, vd + i, 1, vt, cnt + i);
             ta.gt_rgb = gt_dev;
             CKR((launch_tile_m<kModeTrain, false>(c, ta, vt, false, tc)));
           }
+          CKR(run_grad_finalize(c, vd + i, 1, capturing));
           CKR(run_sh_backward(c, vd + i, 1, capturing));
         }
       } else {
         CKR(run_bin(c, vd, n_views, total_tiles, cnt, capturing, pl.groups));
-        CKR(clear_dcolor(c, n_views));
+        CKR(clear_moments(c, n_views));
         {
           StageScope sc(c, kStComposite, capturing);
           TileArgs ta = base_tile_args(c, vd, n_views, total_tiles, cnt);
           ta.gt_rgb = gt_dev;
           CKR((launch_groups<kModeTrain, false>(c, ta, pl.groups)));
         }
+        CKR(run_grad_finalize(c, vd, n_views, capturing));
         CKR(run_sh_backward(c, vd, n_views, capturing));
       }
       if (do_adam) CKR(launch_adam(c, n_cnt, capturing));
@@ -1321,7 +1341,7 @@ int rmesh_get_info(RmeshCtx* c, RmeshInfo* info) {
                    &c->vis_cnt, &c->vis_proj, &c->vis_view, &c->vis_key_alt, &c->vis_val_alt, &c->pair_key,
                    &c->pair_val, &c->pair_key_alt, &c->pair_val_alt, &c->ranges, &c->rgba, &c->aux, &c->dl,
                    &c->gt, &c->out_a, &c->out_b, &c->out_c, &c->out_d, &c->sh, &c->m_sh, &c->v_sh,
-                   &c->vis_color, &c->vis_dcolor, &c->err_in, &c->err_out, &c->aux_data, &c->dl_aux, &c->d_aux,
+                   &c->vis_color, &c->mom, &c->err_in, &c->err_out, &c->aux_data, &c->dl_aux, &c->d_aux,
                    &c->spans_fwd, &c->spans_adj, &c->tile_order, &c->order_hist, &c->tickets};
   for (DevBuf* b : all) info->device_bytes += b->bytes;
   return RMESH_OK;
@@ -1489,7 +1509,8 @@ static int backward_impl(RmeshCtx* c, const float* dl, const float* dl_aux, floa
   CK(cudaMemsetAsync(c->tickets.p, 0, kMaxTileGroups * 4, c->stream));
   const std::vector<TileGroup> one{TileGroup{TileConf{c->last_ts, c->last_wide}, 0u, c->last_tiles}};
   ViewParams* vd = c->views_d.as<ViewParams>();
-  CKR(clear_dcolor(c, 1));
+  CKR(ensure_moments(c, 1));
+  CKR(clear_moments(c, 1));
   {
     StageScope sc(c, kStComposite, false);
     TileArgs ta = base_tile_args(c, vd, 1, c->last_tiles, cnt);
@@ -1507,6 +1528,7 @@ static int backward_impl(RmeshCtx* c, const float* dl, const float* dl_aux, floa
   }
   if (d_aux && with_aux)
     CK(cudaMemcpyAsync(d_aux, c->d_aux.p, (uint64_t)c->M * c->aux_dim * 4, cudaMemcpyDefault, c->stream));
+  CKR(run_grad_finalize(c, vd, 1, false));
   CKR(run_sh_backward(c, vd, 1, false));
   const size_t N = (size_t)c->N, M = (size_t)c->M;
   CKR(ensure_buf(c, c->out_a, 3 * N * 4));
@@ -1552,7 +1574,8 @@ int rmesh_forward_error(RmeshCtx* c, const float* pixel_err, const float* ssim_e
   float* pe = c->err_in.as<float>();
   CK(cudaMemcpyAsync(pe, pixel_err, npix * 4, cudaMemcpyDefault, c->stream));
   CK(cudaMemcpyAsync(pe + npix, ssim_err, npix * 4, cudaMemcpyDefault, c->stream));
-  CK(cudaMemsetAsync(c->err_out.p, 0, M * 18 * 4, c->stream));
+  CKR(ensure_moments(c, 1));
+  CK(cudaMemsetAsync(c->mom.p, 0, M * kErrMom * 4, c->stream));
   Counters* cnt = c->counters_d.as<Counters>();
   CK(cudaMemsetAsync(c->tickets.p, 0, kMaxTileGroups * 4, c->stream));
   const std::vector<TileGroup> one{TileGroup{TileConf{c->last_ts, c->last_wide}, 0u, c->last_tiles}};
@@ -1562,9 +1585,11 @@ int rmesh_forward_error(RmeshCtx* c, const float* pixel_err, const float* ssim_e
     TileArgs ta = base_tile_args(c, vd, 1, c->last_tiles, cnt);
     ta.pixel_err = pe;
     ta.ssim_err = pe + npix;
-    ta.tet_err = c->err_out.as<float>();
-    ta.tet_count = reinterpret_cast<int*>(c->err_out.as<float>() + M * 16);
     CKR((launch_groups<kModeError, false>(c, ta, one)));
+    error_finalize_kernel<<<(unsigned)((M + 255) / 256), 256, 0, c->stream>>>(
+        (int)M, c->mom.as<float>(), c->rec.as<TetRec>(), c->err_out.as<float>(),
+        reinterpret_cast<int*>(c->err_out.as<float>() + M * 16));
+    CKL();
   }
   CK(cudaMemcpyAsync(tet_err, c->err_out.p, M * 16 * 4, cudaMemcpyDefault, c->stream));
   CK(cudaMemcpyAsync(tet_count, c->err_out.as<float>() + M * 16, M * 8, cudaMemcpyDefault, c->stream));

@@ -110,29 +110,34 @@ __device__ __forceinline__ void scanline_tiles(const float px[4], const float py
 
 // Per-(view, visible tet) record consumed by the tile kernel: everything a
 // tile needs about a tet that depends only on the tet and the view, computed
-// once per view instead of once per (tile, tet) pair.  144 bytes (TMA-sized).
+// once per view instead of once per (tile, tet) pair.  128 bytes: one line; the
+// tile kernel copies the first 96, the span kernel reads the last 32.
 //   nrm[f]  inward normal of face f, n = cross(vc - va, vb - va) flipped toward
 //           the opposite vertex, and num = dot(n, va - cam), explicitly rounded
 //           (rasterize_compute.wgsl:301-314, 360-372)
 //   cb      colour + dot(g, cam - v0) (the base colour at the camera, :395-396), density
-//   gm      colour gradient g; w = face flip bits (bit f) | behind (bit 4)
+//   gm      colour gradient g; w = face flip bits (bit f) | behind (bit 4) |
+//           kPlainPlanes: every |n| component is at most 2^58 and every num is 0
+//           or 2^-60 <= |num| <= 2^60, so that with |den| >= 1e-20 the tile
+//           kernel's fused division keeps all its intermediates in range
 //   px, py  pixel-space vertex projections (c.x/c.w+1)*W/2, (1-c.y/c.w)*H/2 (:163-166)
-//   meta    tet id, the entry's own index (its per-view colour-gradient slot)
-struct __align__(16) TetView {
+constexpr uint32_t kPlainPlanes = 1u << 5;
+struct __align__(128) TetView {
   float4 nrm[4];
   float4 cb;
   float4 gm;
   float4 px;
   float4 py;
-  uint4 meta;
 };
+static_assert(sizeof(TetView) == 128, "record layout");
 
-__device__ __forceinline__ void write_tet_view(TetView* dst, const TetRec& r, const float4 col, const ViewParams& V,
-                                               uint32_t tet, uint32_t j) {
+__device__ __forceinline__ void write_tet_view(TetView* dst, const TetRec& r, const float4 col,
+                                               const ViewParams& V) {
   const float4 vs[4] = {r.a, r.b, r.c, r.d};
   const float camx = V.cam[0], camy = V.cam[1], camz = V.cam[2];
   uint32_t flags = 0u;
   TetView out;
+  bool in_range = true;
 #pragma unroll
   for (int f = 0; f < 4; ++f) {
     const float4 va = vs[kFacesH[f][0]], vb = vs[kFacesH[f][1]], vc = vs[kFacesH[f][2]], vo = vs[kFacesH[f][3]];
@@ -146,7 +151,10 @@ __device__ __forceinline__ void write_tet_view(TetView* dst, const TetRec& r, co
       flags |= 1u << f;
     }
     out.nrm[f] = make_float4(nx, ny, nz, dot3x(nx, ny, nz, fs(va.x, camx), fs(va.y, camy), fs(va.z, camz)));
+    const float n_max = fmaxf(fabsf(nx), fmaxf(fabsf(ny), fabsf(nz))), num = fabsf(out.nrm[f].w);
+    in_range = in_range && n_max <= 0x1p58f && (num == 0.0f || (num >= 0x1p-60f && num <= 0x1p60f));
   }
+  if (in_range) flags |= kPlainPlanes;
   const float gx = r.b.w, gy = r.c.w, gz = r.d.w;
   const float boff = dot3x(gx, gy, gz, fs(camx, r.a.x), fs(camy, r.a.y), fs(camz, r.a.z));
   out.cb = make_float4(fa(col.x, boff), fa(col.y, boff), fa(col.z, boff), r.a.w);
@@ -165,7 +173,6 @@ __device__ __forceinline__ void write_tet_view(TetView* dst, const TetRec& r, co
   out.gm = make_float4(gx, gy, gz, __uint_as_float(flags));
   out.px = make_float4(qx[0], qx[1], qx[2], qx[3]);
   out.py = make_float4(qy[0], qy[1], qy[2], qy[3]);
-  out.meta = make_uint4(tet, j, 0u, 0u);
   *dst = out;
 }
 
@@ -367,7 +374,7 @@ __global__ void __launch_bounds__(256, 3) project_kernel(ProjectArgs a) {
     } else {
       col = a.color4[(size_t)a.color_view_stride * view + tet];
     }
-    write_tet_view(a.vis_view + i, r, col, V, tet, (uint32_t)i);
+    write_tet_view(a.vis_view + i, r, col, V);
   }
 }
 

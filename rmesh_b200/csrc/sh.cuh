@@ -5,7 +5,7 @@
 // c the tet centroid and dir = normalize(c - cam).  The reference has no
 // adjoint for it; this kernel is one.  The tile kernel leaves, for every
 // tile-touching (view, tet) entry j, the gradient of the loss with respect to
-// that entry's colour in vis_dcolor[j], j = tet * n_views + view.  One thread
+// that entry's colour in its moments mom[j], j = tet * n_views + view.  One thread
 // per tet then walks the run's views (an entry exists where vis_cnt[j] > 0, the
 // tet touched a tile of that view; its gradients are contiguous), and chains
 // the colour gradient through softplus (math.wgsl:27-33), the SH basis, the
@@ -20,6 +20,7 @@
 #pragma once
 #include "common.cuh"
 #include "project.cuh"
+#include "tile.cuh"
 
 namespace rm {
 
@@ -72,7 +73,7 @@ struct ShBackwardArgs {
   const TetRec* rec;
   const float* sh;           // [M][3][nc] fp32 coefficients (read as f16, as in the forward)
   const uint32_t* vis_cnt;   // [M * n_views] tiles touched by (tet, view) at tet * n_views + view
-  const float4* vis_dcolor;  // [M * n_views] colour gradient per entry
+  const float* mom;          // [M * n_views][kMom] moments per entry, the colour gradient in columns 17..19
   float* d_sh;               // [M][3][nc], accumulated
   float* grad_slot;          // [M][kGradSlot], colour gradient [4..6] and vertices [7..18] accumulated
 };
@@ -112,7 +113,8 @@ __global__ void __launch_bounds__(128, 4) sh_backward_kernel(ShBackwardArgs a) {
   for (int v = 0; v < a.n_views; ++v) {
     const size_t j = (size_t)t * a.n_views + v;
     if (a.vis_cnt[j] == 0u) continue;
-    const float4 dcol = a.vis_dcolor[j];
+    const float4 dm = *reinterpret_cast<const float4*>(a.mom + j * kMom + 16);
+    const float3 dcol = make_float3(dm.y, dm.z, dm.w);
     if (dcol.x == 0.f && dcol.y == 0.f && dcol.z == 0.f) continue;
     float3 cen, dir;
     const float len = sh_direction(r, a.views[v].cam, cen, dir);
