@@ -18,7 +18,7 @@
 //            word: the pixel spans of four rows, pair_spans_kernel) and keep
 //            the pairs that cover a pixel of the strip;
 //   stage    each kept tet's 96-byte render record (face planes, colour,
-//            gradient) comes by TMA bulk copy into the warp's shared memory;
+//            gradient) comes by asynchronous copies into the warp's shared memory;
 //   runs     each tet's covered pixels ("items", row by row) are cut into runs
 //            of at most R, numbered tet-major over the batch; a round is the
 //            next 32 runs, one per lane.  The batch's coverage bits are
@@ -44,6 +44,8 @@
 // the camera, undoes every covered tet (clamping log T at 0) and skips the
 // gradient when the restored transmittance is below 1e-6 (:424-437).
 #pragma once
+#include <type_traits>
+
 #include "common.cuh"
 #include "project.cuh"
 #include "tma.cuh"
@@ -115,9 +117,10 @@ struct StripCfg {
   static constexpr int S = TS / SR;         // strips per tile
   static constexpr int PX = TS * SR;        // pixels per strip (at most 64)
   static constexpr int NPX = (PX + 31) / 32;  // pixels per lane
-  // items per run; sized so that four CTAs of four strips fit an SM's shared memory
-  static constexpr int RMAX = TS == 16 ? 7 : 8;
-  static constexpr int SLOTS = 32 * (RMAX + 1);
+  // items per run, sized for shared memory; run lengths are odd, so that lanes
+  // at the same place of their runs hit distinct banks
+  static constexpr int RMAX = TS == 16 ? 7 : 9;
+  static constexpr int SLOTS = 32 * RMAX;
   static_assert(TS % SR == 0 && PX <= 64, "strip shape");
 };
 
@@ -125,8 +128,7 @@ template <int TS, int SR, bool AUX>
 struct __align__(16) StripSmem {
   using Cfg = StripCfg<TS, SR>;
   float4 rec[kBatch][6];        // render records: nrm[4], cb, gm
-  // per item slot (a run's items are consecutive, padded by one slot per run so
-  // that lanes hit distinct banks).  Forward: (premultiplied rgb, od).  Adjoint
+  // per item slot (a run's items are consecutive).  Forward: (premultiplied rgb, od).  Adjoint
   // and error: .ex = (od, dl.c) -> (t_prev, d_od_state), .tt = (t_min, t_max)
   union {
     float4 item[Cfg::SLOTS];
@@ -144,7 +146,7 @@ struct __align__(16) StripSmem {
   uint32_t qv[2 * kBatch];      //   and entry
   uint32_t bent[AUX ? kBatch : 1];  // the batch's entries
   __align__(8) int16_t rowbase[kBatch][4];  // per (tet, row), one 8-byte store per tet: i0 with i0 + column = run * R + index in run
-  uint64_t bar;
+  uint16_t piece[36];           // combine: first row | tet slot << 8 of each piece, then the end
 };
 
 __device__ __forceinline__ float4 rec_vertex(const TetRec& r, int i) {
@@ -383,13 +385,6 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
   extern __shared__ __align__(16) unsigned char strip_smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   StripSmem<TS, SR, AUX>& s = reinterpret_cast<StripSmem<TS, SR, AUX>*>(strip_smem_raw)[warp];
-  if (lane == 0) {
-    mbar_init(&s.bar, 1);
-    fence_mbar_init();
-  }
-  __syncwarp();
-  uint32_t parity = 0u;
-  bool failed = false;
   const uint32_t n_units = a.n_tiles * (uint32_t)S;
   const uint32_t lanes_le = 0xffffffffu >> (31 - lane);
 
@@ -399,7 +394,7 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
       if (lane == 0) unit = atomicAdd(a.ticket, 1u);
       unit = __shfl_sync(0xffffffffu, unit, 0);
     }
-    if (unit >= n_units || failed) break;
+    if (unit >= n_units) break;
     uint32_t tile = unit / (uint32_t)S;
     const uint32_t strip = unit - tile * (uint32_t)S;
     if (a.persistent && a.tile_order) tile = a.tile_order[tile];
@@ -478,7 +473,6 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
     uint32_t bw = kEmptySpans, bv = 0u, bcum = 0u;
     PMask bmask = 0;
     int bcnt = 0, brun = 0, n_runs = 0, R = 1;
-    uint32_t rmul = 65536u;  // i / R = (i * rmul) >> 16 for every run * R + index of a batch
     uint32_t tmask[NPX];     // tets of the batch covering each of this lane's pixels
     // gathers the next batch, starts its record copies and prepares its runs;
     // returns its number of tets (0: list done)
@@ -508,11 +502,15 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
         s.qv[lane] = v2;
       }
       if (AUX) s.bent[lane] = bv;
-      // records: the warp has read the previous batch's (the caller's barrier)
-      fence_proxy_async_smem();
-      if (lane == 0) mbar_arrive_expect_tx(&s.bar, (uint32_t)nb * 96u);
-      __syncwarp();
-      if (lane < nb) bulk_copy_g2s(&s.rec[lane][0], a.vis_view + bv, 96u, &s.bar);
+      // records (the warp has read the previous batch's): six 16-byte pieces each,
+      // consecutive lanes on consecutive pieces.  Asynchronous copies of a warp are
+      // one instruction for 32 pieces, where a bulk copy per record issues alone.
+#pragma unroll
+      for (int i = 0; i < 6; ++i) {
+        const int c = 32 * i + lane, k = c / 6;
+        const uint32_t entry = __shfl_sync(0xffffffffu, bv, k);
+        if (k < nb) async_copy16(&s.rec[0][0] + c, reinterpret_cast<const float4*>(a.vis_view + entry) + (c - 6 * k));
+      }
       // pixels
       uint32_t width;
       bcum = span_prefix(bw, width, bcnt);
@@ -525,16 +523,17 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
       // run length: the cheapest of a few, a round costing about its longest
       // run plus one item's work for the set-up and the combine
       const int cmax = __reduce_max_sync(0xffffffffu, bcnt);
-      constexpr int kCand[5] = {RMAX, 6, 4, 3, 2};
+      constexpr int kCand[4] = {RMAX, 7, 5, 3};
       int best = 0x7fffffff;
+      uint32_t rmul = 0u;
 #pragma unroll
-      for (int i = 0; i < 5; ++i) {
+      for (int i = 0; i < 4; ++i) {
         const int total = __reduce_add_sync(0xffffffffu, (bcnt + kCand[i] - 1) / kCand[i]);
         const int cost = ((total + 31) >> 5) * (min(kCand[i], cmax) + 1);
         if (cost < best) {
           best = cost;
           R = kCand[i];
-          rmul = (65536u + (uint32_t)kCand[i] - 1u) / (uint32_t)kCand[i];
+          rmul = (65536u + (uint32_t)kCand[i] - 1u) / (uint32_t)kCand[i];  // n / R = n * rmul >> 16 for small n
         }
       }
       const int nr = (int)(((uint32_t)(bcnt + R - 1) * rmul) >> 16);
@@ -557,20 +556,14 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
       }
 #pragma unroll
       for (int q = 0; q < NPX; ++q) tmask[q] = warp_transpose_bits((uint32_t)(bmask >> (q ? 32 : 0)), lane);
-      const bool ok = mbar_wait_bounded(&s.bar, parity, 1u << 20);
-      parity ^= 1u;
-      if (__any_sync(0xffffffffu, !ok)) {
-        failed = true;
-        if (lane == 0) atomicOr(&a.counters->err, kErrSpinTimeout);
-        return 0;
-      }
+      async_copy_wait();
       __syncwarp();
       return nb;
     };
 
     // the round's run of this lane: tet slot, first pixels, number of items;
     // heads: lanes > 0 whose run is the first of its tet (or past the last run)
-    int rk = 0, rk0 = 0, rlen = 0;
+    int rk = 0, rk0 = 0, rklast = 0, rlen = 0;
     uint32_t rentry = 0u;
     PMask rmask = 0;
     unsigned heads = 0u;
@@ -579,6 +572,7 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
       const int d = brun - base;
       heads = __reduce_or_sync(0xffffffffu, d > 0 && d < 32 ? 1u << d : 0u);
       rk = min(rk0 + __popc(heads & lanes_le), kBatch - 1);
+      rklast = __shfl_sync(0xffffffffu, rk, 31);
       const int run0 = __shfl_sync(0xffffffffu, brun, rk);
       const int cnt = __shfl_sync(0xffffffffu, bcnt, rk);
       const uint32_t w = __shfl_sync(0xffffffffu, bw, rk);
@@ -595,7 +589,8 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
     };
     // phase 0: intersection + integral of the run's items.  Colours are clipped
     // at 0 in the forward (rasterize_compute.wgsl:409), at -1e20 in the adjoint (:411).
-    auto phase0 = [&](bool fwd) {
+    auto phase0 = [&](auto forward) {
+      constexpr bool fwd = decltype(forward)::value;
       if (rlen > 0) {
         float4 nrm[4];
 #pragma unroll
@@ -603,7 +598,7 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
         const float4 cb0 = s.rec[rk][4], gg = s.rec[rk][5];
         const bool moved = fwd && has_min_t;  // rays start at min_t
         const bool in_range = (__float_as_uint(gg.w) & kPlainPlanes) && !moved;
-        int slot = lane * (R + 1);
+        int slot = lane * R;
         PMask m = rmask;
 #pragma unroll 1
         for (int j = 0; j < rlen; ++j, ++slot) {
@@ -613,7 +608,7 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
           float t_min, t_max;
           int fmin, fmax;
           bool plain;
-          bool hit = intersect4_plain<(AUX || MODE != kModeForward)>(nrm, d.x, d.y, d.z, t_min, t_max, fmin, fmax, plain);
+          bool hit = intersect4_plain<(AUX || !fwd)>(nrm, d.x, d.y, d.z, t_min, t_max, fmin, fmax, plain);
           if (!(plain && in_range)) {
             float numo[4] = {nrm[0].w, nrm[1].w, nrm[2].w, nrm[3].w};
             if (moved) {
@@ -662,28 +657,65 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
         }
       }
     };
-    // phase 1 item lookup: slot of (tet k, this lane's pixel q) in the round that
-    // starts at run `base`, or -1 when the item belongs to a later round
-    auto slot_of = [&](int k, int q, int base) -> int {
-      const int p = 32 * q + lane;
-      const int row = p / TS, col = p - (p / TS) * TS;
-      const int i = (int)s.rowbase[k][row & 3] + col;
-      const int run = (int)(((uint32_t)i * rmul) >> 16);
-      return run < base + 32 ? i + run - base * (R + 1) : -1;
+    // phase 1: the round's tets of pixel q (taken out of tmask).  Only the tet of
+    // the round's last run may continue in the next round: its item at this pixel
+    // is looked up once.
+    auto take_tets = [&](int q, int base, bool on) -> uint32_t {
+      const int row = (32 * q + lane) / TS & 3, col = (32 * q + lane) % TS;
+      uint32_t m = on ? tmask[q] & ((2u << rklast) - 1u) : 0u;
+      if ((m >> rklast) & 1u) {
+        if ((int)s.rowbase[rklast][row] + col >= (base + 32) * R) m ^= 1u << rklast;
+      }
+      tmask[q] &= ~m;
+      return m;
     };
-    // adds the lanes' rows (columns 0..NC-1, one lane per run) to `dst` per tet:
-    // lane c sums column c over each tet's adjacent rows.  Column kMaxCol, when
-    // it is one, holds integers and keeps their maximum.
-    auto combine = [&](int base, float* dst, int stride, int cols, int max_col) {
+    // slot of (tet k, this lane's pixel q) in the round that starts at run `base`
+    auto slot_of = [&](int k, int q, int base) -> int {
+      const int row = (32 * q + lane) / TS & 3, col = (32 * q + lane) % TS;
+      return (int)s.rowbase[k][row] + (col - base * R);
+    };
+    // adds the lanes' rows (one per run) to `dst` per tet.  The rows are cut into
+    // pieces of one tet and at most eight rows; six lanes (four columns each) take
+    // a piece, five pieces at a time, and add its sums with 16-byte atomics.
+    auto combine = [&](int base, float* dst) {
+      static_assert(kMom == 24, "six lanes of four columns");
+      const int n_rows = min(32, n_runs - base);
+      const unsigned cuts = (heads | 0x01010101u) & (0xffffffffu >> (32 - n_rows));
+      if ((cuts >> lane) & 1u) s.piece[__popc(cuts & (lanes_le >> 1))] = (uint16_t)(lane | (rk << 8));
+      const int n_pieces = __popc(cuts);
+      if (lane == 0) s.piece[n_pieces] = (uint16_t)n_rows;
+      __syncwarp();
+      const int sub = lane / 6, col = 4 * (lane - 6 * sub);
+      for (int i0 = 0; i0 < n_pieces; i0 += 5) {
+        const int i = i0 + sub;
+        const bool on = lane < 30 && i < n_pieces;
+        const uint32_t pc = on ? s.piece[i] : 0u;
+        const uint32_t entry = __shfl_sync(0xffffffffu, bv, (int)(pc >> 8));
+        if (on) {
+          const int r1 = (int)(s.piece[i + 1] & 255u);
+          int r = (int)(pc & 255u);
+          float4 sum = *reinterpret_cast<const float4*>(&s.red[r][col]);
+          for (++r; r < r1; ++r) {
+            const float4 v = *reinterpret_cast<const float4*>(&s.red[r][col]);
+            sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+          }
+          if (sum.x != 0.0f || sum.y != 0.0f || sum.z != 0.0f || sum.w != 0.0f)
+            atomicAdd(reinterpret_cast<float4*>(dst + (size_t)entry * kMom + col), sum);
+        }
+      }
+    };
+    // the same for the error statistics: lane c sums column c over each tet's
+    // adjacent rows, the last column (integers) by maximum
+    auto combine_error = [&](int base, float* dst) {
       const int n_rows = min(32, n_runs - base);
       int k = rk0;
-      for (int r0 = 0; r0 < n_rows; ++k) {  // one tet segment [r0, r1) at a time
+      for (int r0 = 0; r0 < n_rows; ++k) {  // one tet's rows [r0, r1) at a time
         const unsigned later = heads & ~((2u << r0) - 1u);
         const int r1 = later ? min(__ffs(later) - 1, n_rows) : n_rows;
         const uint32_t entry = __shfl_sync(0xffffffffu, bv, k);
-        if (lane < cols) {
-          float* at = dst + (size_t)entry * (size_t)stride + lane;
-          if (lane == max_col) {
+        if (lane < kErrMom) {
+          float* at = dst + (size_t)entry * kErrMom + lane;
+          if (lane == kErrMom - 1) {
             int mx = 0;
             for (int r = r0; r < r1; ++r) mx = max(mx, __float_as_int(s.red[r][lane]));
             if (mx > 0) atomicMax(reinterpret_cast<int*>(at), mx);
@@ -704,10 +736,8 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
     // =============== forward (front to back) ===============
     if (MODE == kModeForward || MODE == kModeTrain) {
       float nd[AUX ? NPX : 1][4], en[AUX ? NPX : 1][4];
-      bool alive[NPX];
 #pragma unroll
       for (int q = 0; q < NPX; ++q) {
-        alive[q] = valid[q];
         if (AUX) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) nd[q][i] = en[q][i] = 0.0f;
@@ -723,70 +753,76 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
         if (nb == 0) break;
         for (int base = 0; base < n_runs; base += 32) {
           take_runs(base);
-          phase0(true);
+          phase0(std::true_type{});
           __syncwarp();
-          // phase 1: composite each pixel's items nearest first
+          // phase 1: composite each pixel's items nearest first.  The lane's pixels
+          // advance together (two chains in flight) and without branches: an item
+          // that does not count (ray miss, T below the cut) has weight 0.
+          uint32_t m[NPX], any = 0u;
 #pragma unroll
           for (int q = 0; q < NPX; ++q) {
-            uint32_t m = alive[q] ? tmask[q] : 0u;
-            while (m) {
-              if (logT[q] < -13.8f) {
-                alive[q] = false;
-                break;
-              }
-              const int k = __ffs(m) - 1;
-              const int slot = slot_of(k, q, base);
-              if (slot < 0) break;
-              m &= m - 1u;
+            m[q] = take_tets(q, base, true);
+            if (logT[q] < -13.8f) m[q] = 0u;
+            any |= m[q];
+          }
+          while (any) {
+            any = 0u;
+#pragma unroll
+            for (int q = 0; q < NPX; ++q) {
+              const bool has = m[q] != 0u;
+              const int k = (__ffs(m[q]) - 1) & 31;
+              const int slot = has ? slot_of(k, q, base) : 0;
+              m[q] &= m[q] - 1u;
               const float4 c = s.item[slot];
-              if (c.w < 0.0f) continue;  // ray miss
               const float Tj = exp_fast(fmaxf(logT[q], -88.0f));
-              if (Tj >= 1e-6f) {
-                Cr[q] += c.x * Tj; Cg[q] += c.y * Tj; Cb[q] += c.z * Tj;
-                logT[q] -= c.w;
-                if (AUX) {
-                  const float2 c2 = s.aux[slot];
-                  const float t_min = c2.x, t_max = c2.y;
-                  const int entry = (int)(s.pk[slot] & 7u);
-                  const float od = c.w;
-                  const float alpha_t = exp_fast(-od);  // as the intersection phase computed it
-                  const float ph = fabsf(od) < 0.02f
-                                       ? 1.0f + od * (-0.5f + od * (1.0f / 6.0f + od * (-1.0f / 24.0f)))
-                                       : clipf(__fdividef(1.0f - alpha_t, od), kMinVal, kMaxVal);
-                  const float w0 = ph - alpha_t, w1 = 1.0f - ph;
-                  const float alpha = 1.0f - alpha_t;
-                  float enx = 0.f, eny = 0.f, enz = 0.f;
-                  if (entry < 4) {
-                    const float4 n = s.rec[k][entry];
-                    const float l = sqrtf(n.x * n.x + n.y * n.y + n.z * n.z);
-                    enx = -n.x / l; eny = -n.y / l; enz = -n.z / l;
-                  }
-                  const float ta = Tj * alpha;
-                  nd[q][0] += ta * enx; nd[q][1] += ta * eny; nd[q][2] += ta * enz;
-                  nd[q][3] += Tj * (w0 * t_max + w1 * t_min);
-                  const float wt = alpha * Tj;
-                  const float cmid = (t_min + t_max) * 0.5f;
-                  const float wc = wt * cmid;
-                  en[q][0] += wt;
-                  en[q][1] += wt > 1e-20f ? wt * logf(wt) : 0.0f;
-                  en[q][2] += wt * cmid;
-                  en[q][3] += wc > 1e-20f ? wc * logf(wc) : 0.0f;
-                  if (a.aux_dim > 0) {
-                    const float* ad = a.aux_data + (size_t)(s.bent[k] / (uint32_t)a.n_views) * a.aux_dim;
-                    float* aux_px = a.aux + pix[q] * (size_t)(8 + a.aux_dim) + 8;
-                    for (int ai = 0; ai < a.aux_dim; ++ai) aux_px[ai] += ta * ad[ai];
-                  }
+              const bool on = has && c.w >= 0.0f && Tj >= 1e-6f;
+              const float w = on ? Tj : 0.0f;
+              Cr[q] += c.x * w; Cg[q] += c.y * w; Cb[q] += c.z * w;
+              logT[q] -= on ? c.w : 0.0f;
+              if (logT[q] < -13.8f) m[q] = 0u;  // saturated: the rest is skipped
+              any |= m[q];
+              if (AUX) {
+                if (!on) continue;
+                const float2 c2 = s.aux[slot];
+                const float t_min = c2.x, t_max = c2.y;
+                const int entry = (int)(s.pk[slot] & 7u);
+                const float od = c.w;
+                const float alpha_t = exp_fast(-od);  // as the intersection phase computed it
+                const float ph = fabsf(od) < 0.02f
+                                     ? 1.0f + od * (-0.5f + od * (1.0f / 6.0f + od * (-1.0f / 24.0f)))
+                                     : clipf(__fdividef(1.0f - alpha_t, od), kMinVal, kMaxVal);
+                const float w0 = ph - alpha_t, w1 = 1.0f - ph;
+                const float alpha = 1.0f - alpha_t;
+                float enx = 0.f, eny = 0.f, enz = 0.f;
+                if (entry < 4) {
+                  const float4 n = s.rec[k][entry];
+                  const float l = sqrtf(n.x * n.x + n.y * n.y + n.z * n.z);
+                  enx = -n.x / l; eny = -n.y / l; enz = -n.z / l;
+                }
+                const float ta = Tj * alpha;
+                nd[q][0] += ta * enx; nd[q][1] += ta * eny; nd[q][2] += ta * enz;
+                nd[q][3] += Tj * (w0 * t_max + w1 * t_min);
+                const float wt = alpha * Tj;
+                const float cmid = (t_min + t_max) * 0.5f;
+                const float wc = wt * cmid;
+                en[q][0] += wt;
+                en[q][1] += wt > 1e-20f ? wt * logf(wt) : 0.0f;
+                en[q][2] += wt * cmid;
+                en[q][3] += wc > 1e-20f ? wc * logf(wc) : 0.0f;
+                if (a.aux_dim > 0) {
+                  const float* ad = a.aux_data + (size_t)(s.bent[k] / (uint32_t)a.n_views) * a.aux_dim;
+                  float* aux_px = a.aux + pix[q] * (size_t)(8 + a.aux_dim) + 8;
+                  for (int ai = 0; ai < a.aux_dim; ++ai) aux_px[ai] += ta * ad[ai];
                 }
               }
             }
-            tmask[q] = m;
           }
           __syncwarp();
         }
         // all pixels saturated: the remaining tets would all be skipped
         bool more = false;
 #pragma unroll
-        for (int q = 0; q < NPX; ++q) more = more || (alive[q] && logT[q] >= -13.8f);
+        for (int q = 0; q < NPX; ++q) more = more || (valid[q] && logT[q] >= -13.8f);
         if (!__any_sync(0xffffffffu, more)) break;
       }
 #pragma unroll
@@ -830,16 +866,15 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
         if (nb == 0) break;
         for (int base = 0; base < n_runs; base += 32) {
           take_runs(base);
-          phase0(true);
+          phase0(std::true_type{});
           __syncwarp();
 #pragma unroll
           for (int q = 0; q < NPX; ++q) {
-            uint32_t m = alive[q] ? tmask[q] : 0u;
+            uint32_t m = take_tets(q, base, alive[q]);
             while (m) {
               if (logT[q] < -5.5f) break;
               const int k = __ffs(m) - 1;
               const int slot = slot_of(k, q, base);
-              if (slot < 0) break;
               m &= m - 1u;
               const float od = s.a.ex[slot].x;
               if (od < 0.0f) continue;  // ray miss
@@ -849,7 +884,6 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
                 logT[q] -= od;
               }
             }
-            tmask[q] = m;
             if (logT[q] < -5.5f) alive[q] = false;
           }
           __syncwarp();
@@ -858,7 +892,7 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
 #pragma unroll
           for (int i = 0; i < kErrMom; ++i) acc[i] = 0.0f;
           int mx = 0;
-          for (int j = 0, slot = lane * (R + 1); j < rlen; ++j, ++slot) {
+          for (int j = 0, slot = lane * R; j < rlen; ++j, ++slot) {
             const float2 st = s.a.ex[slot];
             if (!(st.y > 0.5f)) continue;
             const float2 ix = s.a.tt[slot];
@@ -880,7 +914,7 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
 #pragma unroll
           for (int i = 0; i < kErrMom; ++i) s.red[lane][i] = acc[i];
           __syncwarp();
-          combine(base, a.mom, kErrMom, kErrMom, kErrMom - 1);
+          combine_error(base, a.mom);
           __syncwarp();
         }
         bool more = false;
@@ -937,35 +971,45 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
       }
       __syncwarp();
       start_list(false);
-      while (!failed) {
+      while (true) {
         // adjoint: edge crossings only (backward_tiled_compute.wgsl:241-299)
         const int nb = next_batch(false);
         if (nb == 0) break;
         for (int base = 0; base < n_runs; base += 32) {
           take_runs(base);
-          phase0(false);
+          phase0(std::false_type{});
           __syncwarp();
-          // phase 1: undo each pixel's items farthest first
+          // phase 1: undo each pixel's items farthest first, the lane's pixels
+          // together; the item gets (t_prev, d_od_state), with t_prev 0 where it has
+          // no gradient, and a ray miss changes nothing
+          uint32_t m[NPX], any = 0u;
 #pragma unroll
           for (int q = 0; q < NPX; ++q) {
-            uint32_t m = valid[q] ? tmask[q] : 0u;
-            while (m) {
-              const int k = __ffs(m) - 1;
+            m[q] = take_tets(q, base, true);
+            any |= m[q];
+          }
+          while (any) {
+            any = 0u;
+#pragma unroll
+            for (int q = 0; q < NPX; ++q) {
+              const bool has = m[q] != 0u;
+              const int k = (__ffs(m[q]) - 1) & 31;
               const int slot = slot_of(k, q, base);
-              if (slot < 0) break;
-              m &= m - 1u;
-              const float2 c = s.a.ex[slot];
-              if (c.x < 0.0f) continue;  // ray miss: no state change, no gradient
+              m[q] &= m[q] - 1u;
+              any |= m[q];
+              float2 c = make_float2(-1.0f, 0.0f);
+              if (has) c = s.a.ex[slot];
+              const bool hit = c.x >= 0.0f;
               const float prev_logT = fminf(logT[q] + c.x, 0.0f);
               const float t_prev = exp_fast(fmaxf(prev_logT, -88.0f));
-              logT[q] = prev_logT;
-              float2 st = make_float2(0.0f, 0.0f);  // no gradient
-              if (t_prev >= 1e-6f) {
-                // custom aux channels (aux += T alpha a[tet], rasterize_compute.wgsl:458-462)
-                // continue the transmittance chain like a colour alpha a[tet]:
-                // aux_s = sum_ai dl_aux[pixel][ai] a[tet][ai]
-                float aux_w = 0.0f;
-                if (AUX && MODE == kModeBackward && a.dl_aux) {
+              logT[q] = hit ? prev_logT : logT[q];
+              const bool on = hit && t_prev >= 1e-6f;
+              float aux_w = 0.0f;
+              if (AUX && MODE == kModeBackward) {
+                if (on && a.dl_aux) {
+                  // custom aux channels (aux += T alpha a[tet], rasterize_compute.wgsl:458-462)
+                  // continue the transmittance chain like a colour alpha a[tet]:
+                  // aux_s = sum_ai dl_aux[pixel][ai] a[tet][ai]
                   float aux_s = 0.0f;
                   const float* dla = a.dl_aux + pix[q] * (size_t)a.aux_dim;
                   const float* ad = a.aux_data + (size_t)(s.bent[k] / (uint32_t)a.n_views) * a.aux_dim;
@@ -973,12 +1017,11 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
                   aux_w = (1.0f - exp_fast(-c.x)) * aux_s;  // alpha * aux_s
                   s.aux[slot].x = aux_s;
                 }
-                st = make_float2(t_prev, -dlogT[q]);
-                dlogT[q] = clipf(dlogT[q] + (c.y + aux_w) * t_prev, kMinVal, kMaxVal);
               }
-              s.a.ex[slot] = st;
+              if (has) s.a.ex[slot] = make_float2(on ? t_prev : 0.0f, -dlogT[q]);
+              const float next = clipf(dlogT[q] + (c.y + aux_w) * t_prev, kMinVal, kMaxVal);
+              dlogT[q] = on ? next : dlogT[q];
             }
-            tmask[q] = m;
           }
           __syncwarp();
           // phase 2: per-item adjoint over the run.
@@ -1001,7 +1044,7 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
           if (rlen > 0) {
             const float4 cb = s.rec[rk][4], gg = s.rec[rk][5];
             const uint32_t flips = __float_as_uint(gg.w);
-            int slot = lane * (R + 1);
+            int slot = lane * R;
 #pragma unroll 1
             for (int j = 0; j < rlen; ++j, ++slot) {
               // (t_prev, d_od_state); ray misses and items below the transmittance
@@ -1088,7 +1131,7 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
           fac[4] = make_float4(acc[0], acc[1], acc[2], acc[3]);
           fac[5] = make_float4(acc[4], acc[5], acc[6], acc[7]);
           __syncwarp();
-          combine(base, a.mom, kMom, kMom, -1);
+          combine(base, a.mom);
           __syncwarp();
         }
       }
