@@ -70,6 +70,8 @@ constexpr int kErrMom = 12;
 constexpr int kRedCols = 28;
 constexpr int kStripWarps = 4;  // warps (independent strips) per CTA
 
+constexpr int kAuxShared = 8;   // custom aux channels accumulated in shared memory
+
 enum TileMode : int { kModeForward = 0, kModeBackward = 1, kModeTrain = 2, kModeError = 3 };
 
 struct TileArgs {
@@ -138,7 +140,9 @@ struct __align__(16) StripSmem {
     } a;
   };
   __align__(16) float red[32][kRedCols];  // per-lane moment rows of phase 2
-  float2 aux[AUX ? Cfg::SLOTS : 2];  // forward: (t_min, t_max); backward: .x = aux_s
+  // forward: (t_min, t_max); backward: (aux_s, d a[tet] weight T_prev alpha)
+  float2 aux[AUX ? Cfg::SLOTS : 2];
+  float caux[AUX ? kAuxShared * Cfg::PX : 4];  // forward: the pixels' first custom channels
   uint16_t pk[Cfg::SLOTS];      // pack_item
   float4 pdir[Cfg::PX];         // pixel ray direction; w: the pixel's dL/dR (adjoint)
   float2 pdl[Cfg::PX];          // the pixel's dL/dG, dL/dB (adjoint); pixel and SSIM error (error mode)
@@ -417,6 +421,12 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
     // adjoint keeps the origin at the camera (backward_tiled_compute.wgsl:377)
     const bool has_min_t = V.min_t != 0.0f;
 
+    // image index of strip pixel p
+    auto strip_pixel = [&](int p) -> size_t {
+      const int row = p / TS, col = p - (p / TS) * TS;
+      return (size_t)V.pix_base + (size_t)(y0 + (uint32_t)row) * (size_t)V.W + (size_t)(x0 + (uint32_t)col);
+    };
+
     // this lane's pixels p = 32 q + lane
     bool valid[NPX];
     size_t pix[NPX];
@@ -650,7 +660,19 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
             }
           } else {
             const float2 dgb = s.pdl[p];
-            s.a.ex[slot] = make_float2(out.w, d.w * out.x + dgb.x * out.y + dgb.y * out.z);
+            float dlc = d.w * out.x + dgb.x * out.y + dgb.y * out.z;
+            if (AUX && MODE == kModeBackward) {
+              // custom aux channels (aux += T alpha a[tet], rasterize_compute.wgsl:458-462)
+              // continue the transmittance chain like a colour alpha a[tet]:
+              // aux_s = sum_ai dl_aux[pixel][ai] a[tet][ai]
+              const float* dla = a.dl_aux + strip_pixel(p) * (size_t)a.aux_dim;
+              const float* ad = a.aux_data + (size_t)(rentry / (uint32_t)a.n_views) * a.aux_dim;
+              float aux_s = 0.0f;
+              for (int ai = 0; ai < a.aux_dim; ++ai) aux_s += dla[ai] * ad[ai];
+              dlc += (1.0f - I.alpha_t) * aux_s;
+              s.aux[slot] = make_float2(aux_s, 0.0f);
+            }
+            s.a.ex[slot] = make_float2(out.w, dlc);
             s.a.tt[slot] = out_t;
             s.pk[slot] = (uint16_t)out_p;
           }
@@ -741,10 +763,12 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
         if (AUX) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) nd[q][i] = en[q][i] = 0.0f;
-          // custom aux channels accumulate in place in the output row of the pixel
-          // (rasterize_compute.wgsl:458-462), so they start at zero
-          if (a.aux && valid[q])
-            for (int ai = 0; ai < a.aux_dim; ++ai) a.aux[pix[q] * (size_t)(8 + a.aux_dim) + 8 + ai] = 0.0f;
+          // custom aux channels (rasterize_compute.wgsl:458-462): the first accumulate
+          // in shared memory, the others in place in the pixel's output row
+          if (valid[q]) {
+            for (int ai = 0; ai < kAuxShared; ++ai) s.caux[ai * PX + 32 * q + lane] = 0.0f;
+            for (int ai = kAuxShared; ai < a.aux_dim; ++ai) a.aux[pix[q] * (size_t)(8 + a.aux_dim) + 8 + ai] = 0.0f;
+          }
         }
       }
       start_list(true);
@@ -796,8 +820,8 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
                 float enx = 0.f, eny = 0.f, enz = 0.f;
                 if (entry < 4) {
                   const float4 n = s.rec[k][entry];
-                  const float l = sqrtf(n.x * n.x + n.y * n.y + n.z * n.z);
-                  enx = -n.x / l; eny = -n.y / l; enz = -n.z / l;
+                  const float l = -rsqrtf(n.x * n.x + n.y * n.y + n.z * n.z);
+                  enx = n.x * l; eny = n.y * l; enz = n.z * l;
                 }
                 const float ta = Tj * alpha;
                 nd[q][0] += ta * enx; nd[q][1] += ta * eny; nd[q][2] += ta * enz;
@@ -812,7 +836,9 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
                 if (a.aux_dim > 0) {
                   const float* ad = a.aux_data + (size_t)(s.bent[k] / (uint32_t)a.n_views) * a.aux_dim;
                   float* aux_px = a.aux + pix[q] * (size_t)(8 + a.aux_dim) + 8;
-                  for (int ai = 0; ai < a.aux_dim; ++ai) aux_px[ai] += ta * ad[ai];
+                  const int n_sh = min(a.aux_dim, kAuxShared);
+                  for (int ai = 0; ai < n_sh; ++ai) s.caux[ai * PX + 32 * q + lane] += ta * ad[ai];
+                  for (int ai = kAuxShared; ai < a.aux_dim; ++ai) aux_px[ai] += ta * ad[ai];
                 }
               }
             }
@@ -840,6 +866,7 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
               o[i] = nd[q][i];
               o[4 + i] = en[q][i];
             }
+            for (int ai = 0; ai < min(a.aux_dim, kAuxShared); ++ai) o[8 + ai] = s.caux[ai * PX + 32 * q + lane];
           }
         }
       }
@@ -1004,22 +1031,8 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
               const float t_prev = exp_fast(fmaxf(prev_logT, -88.0f));
               logT[q] = hit ? prev_logT : logT[q];
               const bool on = hit && t_prev >= 1e-6f;
-              float aux_w = 0.0f;
-              if (AUX && MODE == kModeBackward) {
-                if (on && a.dl_aux) {
-                  // custom aux channels (aux += T alpha a[tet], rasterize_compute.wgsl:458-462)
-                  // continue the transmittance chain like a colour alpha a[tet]:
-                  // aux_s = sum_ai dl_aux[pixel][ai] a[tet][ai]
-                  float aux_s = 0.0f;
-                  const float* dla = a.dl_aux + pix[q] * (size_t)a.aux_dim;
-                  const float* ad = a.aux_data + (size_t)(s.bent[k] / (uint32_t)a.n_views) * a.aux_dim;
-                  for (int ai = 0; ai < a.aux_dim; ++ai) aux_s += dla[ai] * ad[ai];
-                  aux_w = (1.0f - exp_fast(-c.x)) * aux_s;  // alpha * aux_s
-                  s.aux[slot].x = aux_s;
-                }
-              }
               if (has) s.a.ex[slot] = make_float2(on ? t_prev : 0.0f, -dlogT[q]);
-              const float next = clipf(dlogT[q] + (c.y + aux_w) * t_prev, kMinVal, kMaxVal);
+              const float next = clipf(dlogT[q] + c.y * t_prev, kMinVal, kMaxVal);
               dlogT[q] = on ? next : dlogT[q];
             }
           }
@@ -1073,19 +1086,11 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
               const float d_od_int = dcpr * (I.cer * dw0 + I.csr * dw1) + dcpg * (I.ceg * dw0 + I.csg * dw1) +
                                      dcpb * (I.ceb * dw0 + I.csb * dw1);
               float d_od_aux = 0.0f;
-              if (AUX && MODE == kModeBackward && a.dl_aux) {
+              if (AUX && MODE == kModeBackward) {
                 // the aux channels' own terms: d od += T_prev alpha_t aux_s (d alpha / d od =
-                // alpha_t); d a[tet][ai] += dl_aux[pixel][ai] T_prev alpha
+                // alpha_t); d a[tet][ai] += dl_aux[pixel][ai] T_prev alpha, below
                 d_od_aux = t_prev * I.alpha_t * s.aux[slot].x;
-                const int pr = p / TS, pc = p - (p / TS) * TS;
-                const size_t gp = (size_t)V.pix_base + (size_t)(y0 + (uint32_t)pr) * (size_t)V.W + (size_t)(x0 + (uint32_t)pc);
-                const float* dla = a.dl_aux + gp * (size_t)a.aux_dim;
-                float* dst = a.d_aux + (size_t)(rentry / (uint32_t)a.n_views) * a.aux_dim;
-                const float wa = t_prev * (1.0f - I.alpha_t);
-                for (int ai = 0; ai < a.aux_dim; ++ai) {
-                  const float v = dla[ai] * wa;
-                  if (v != 0.0f) atomicAdd(dst + ai, v);
-                }
+                s.aux[slot].y = t_prev * (1.0f - I.alpha_t);
               }
               const float d_od = clipf(d_od_state + d_od_int + d_od_aux, kMinVal, kMaxVal);
               const bool active = (I.od_raw >= 1e-8f) && (I.od_raw <= 88.0f);
@@ -1126,6 +1131,23 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
                 v.w += st_ * d.z;
                 fac[f] = v;
               }
+            }
+          }
+          if (AUX && MODE == kModeBackward && rlen > 0) {
+            // the run's aux data gradient, four channels at a time
+            float* dst = a.d_aux + (size_t)(rentry / (uint32_t)a.n_views) * a.aux_dim;
+            for (int a0 = 0; a0 < a.aux_dim; a0 += 4) {
+              float sum[4] = {0.f, 0.f, 0.f, 0.f};
+              for (int j = 0, slot = lane * R; j < rlen; ++j, ++slot) {
+                const float wa = s.aux[slot].y;
+                const float* dla = a.dl_aux + strip_pixel((int)(s.pk[slot] >> 5)) * (size_t)a.aux_dim + a0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                  if (a0 + i < a.aux_dim) sum[i] += dla[i] * wa;
+              }
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                if (a0 + i < a.aux_dim && sum[i] != 0.0f) atomicAdd(dst + a0 + i, sum[i]);
             }
           }
           fac[4] = make_float4(acc[0], acc[1], acc[2], acc[3]);
