@@ -677,17 +677,41 @@ int launch_tile_t(RmeshCtx* c, TileArgs& ta, uint32_t n_tiles, bool persistent) 
   return RMESH_OK;
 }
 
+// Rows per strip (4, 2 or 1) of a launch.  A strip is one warp's serial work, so
+// small launches take thinner strips until the chip has a few strips per
+// resident warp; thin strips repeat the per-tet set-up more often and fill fewer
+// pixel lanes.  Measured with 12-pixel tiles (tile kernel, 4 / 2 / 1 rows, in
+// units of 4-row strips per resident warp):
+//   forward + adjoint  2.3: 0.351 / 0.263 / 0.326 ms   2.5: 1.18 / 0.64 / 0.67 ms
+//                      4.3: 0.843 / 0.784 / 1.056 ms   9.4: 2.28 / 2.48 / 3.33 ms
+//                      79: 32.0 / 35.1 / 46.9 ms
+//   forward            0.6: 0.106 / 0.066 / 0.050 ms   8.1: 0.432 / 0.402 / 0.544 ms
+//                      45: 3.18 / 3.13 / 4.47 ms
+// The forward has little set-up and never gains from the four rows.  A wide
+// configuration (twice the threads per tile) takes one step thinner.
+int strip_rows(const RmeshCtx* c, uint32_t n_tiles, TileConf tc, bool adjoint) {
+  const uint64_t strips4 = (uint64_t)n_tiles * (uint64_t)(tc.ts / 4);
+  const uint64_t warps = (uint64_t)c->num_sms * 16u;
+  const int rows = strips4 < warps ? 1 : (!adjoint || strips4 < 6 * warps ? 2 : 4);
+  return tc.wide ? std::max(1, rows / 2) : rows;
+}
+
+template <int TS, int MODE, bool AUX>
+int launch_tile_s(RmeshCtx* c, TileArgs& ta, uint32_t n_tiles, bool persistent, TileConf tc) {
+  switch (strip_rows(c, n_tiles, tc, MODE == kModeBackward || MODE == kModeTrain)) {
+    case 1: return launch_tile_t<TS, 1, MODE, AUX>(c, ta, n_tiles, persistent);
+    case 2: return launch_tile_t<TS, 2, MODE, AUX>(c, ta, n_tiles, persistent);
+    default: return launch_tile_t<TS, 4, MODE, AUX>(c, ta, n_tiles, persistent);
+  }
+}
+
 // one launch over the tiles of a group (ta.tile_lo, ta.ticket set by the caller)
 template <int MODE, bool AUX>
 int launch_tile_m(RmeshCtx* c, TileArgs& ta, uint32_t n_tiles, bool persistent, TileConf tc) {
-  const int key = tc.ts * 2 + (tc.wide ? 1 : 0);
-  switch (key) {
-    case 16: return launch_tile_t<8, 4, MODE, AUX>(c, ta, n_tiles, persistent);
-    case 17: return launch_tile_t<8, 2, MODE, AUX>(c, ta, n_tiles, persistent);
-    case 24: return launch_tile_t<12, 4, MODE, AUX>(c, ta, n_tiles, persistent);
-    case 25: return launch_tile_t<12, 2, MODE, AUX>(c, ta, n_tiles, persistent);
-    case 32: return launch_tile_t<16, 4, MODE, AUX>(c, ta, n_tiles, persistent);
-    case 33: return launch_tile_t<16, 2, MODE, AUX>(c, ta, n_tiles, persistent);
+  switch (tc.ts) {
+    case 8: return launch_tile_s<8, MODE, AUX>(c, ta, n_tiles, persistent, tc);
+    case 12: return launch_tile_s<12, MODE, AUX>(c, ta, n_tiles, persistent, tc);
+    case 16: return launch_tile_s<16, MODE, AUX>(c, ta, n_tiles, persistent, tc);
     default: return fail(c, RMESH_ERR_INVALID_ARG, "tile size must be 8, 12 or 16");
   }
 }
@@ -742,12 +766,11 @@ int clear_moments(RmeshCtx* c, int n_views) {
 }
 
 // the tets' gradients from an adjoint launch's moments
-int run_grad_finalize(RmeshCtx* c, const ViewParams* views_dev, int n_views, bool capturing) {
+int run_grad_finalize(RmeshCtx* c, int n_views, bool capturing) {
   StageScope sc(c, kStComposite, capturing);
   GradFinalizeArgs ga;
   ga.M = (int)c->M;
   ga.n_views = n_views;
-  ga.views = views_dev;
   ga.rec = c->rec.as<TetRec>();
   ga.vis_cnt = c->vis_cnt.as<uint32_t>();
   ga.mom = c->mom.as<float>();
@@ -912,7 +935,7 @@ int train_views(RmeshCtx* c, const RmeshCamera* cams, int n_views, const float* 
             ta.gt_rgb = gt_dev;
             CKR((launch_tile_m<kModeTrain, false>(c, ta, vt, false, tc)));
           }
-          CKR(run_grad_finalize(c, vd + i, 1, capturing));
+          CKR(run_grad_finalize(c, 1, capturing));
           CKR(run_sh_backward(c, vd + i, 1, capturing));
         }
       } else {
@@ -924,7 +947,7 @@ int train_views(RmeshCtx* c, const RmeshCamera* cams, int n_views, const float* 
           ta.gt_rgb = gt_dev;
           CKR((launch_groups<kModeTrain, false>(c, ta, pl.groups)));
         }
-        CKR(run_grad_finalize(c, vd, n_views, capturing));
+        CKR(run_grad_finalize(c, n_views, capturing));
         CKR(run_sh_backward(c, vd, n_views, capturing));
       }
       if (do_adam) CKR(launch_adam(c, n_cnt, capturing));
@@ -1528,7 +1551,7 @@ static int backward_impl(RmeshCtx* c, const float* dl, const float* dl_aux, floa
   }
   if (d_aux && with_aux)
     CK(cudaMemcpyAsync(d_aux, c->d_aux.p, (uint64_t)c->M * c->aux_dim * 4, cudaMemcpyDefault, c->stream));
-  CKR(run_grad_finalize(c, vd, 1, false));
+  CKR(run_grad_finalize(c, 1, false));
   CKR(run_sh_backward(c, vd, 1, false));
   const size_t N = (size_t)c->N, M = (size_t)c->M;
   CKR(ensure_buf(c, c->out_a, 3 * N * 4));

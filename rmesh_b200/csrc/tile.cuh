@@ -60,8 +60,8 @@ __device__ __forceinline__ uint8_t pack_span(short2 sp) {
   return sp.x > sp.y ? (uint8_t)0xF0u : (uint8_t)((sp.x << 4) | sp.y);
 }
 // Moments per entry, summed over its items (see phase 2): columns 4f..4f+3 hold
-// (S, P.x, P.y, P.z) of face f, 16 density, 17..19 colour, 20 sum(sb),
-// 21..23 d * d(dc/dt).
+// (S, P.x, P.y, P.z) of face f, 16 density, 17..19 colour, 20 the sum of the three
+// colour gradients, 21..23 the colour gradient's gradient.
 constexpr int kMom = 24;
 // error statistics per tet: 11 sums and a maximum
 constexpr int kErrMom = 12;
@@ -113,7 +113,7 @@ struct TileArgs {
   uint32_t* ticket;  // persistent strip-queue head of this launch (zeroed before it)
 };
 
-// Strips of a tile: SR rows of TS pixels.
+// Strips of a tile: SR rows (1, 2 or 4) of TS pixels.
 template <int TS, int SR>
 struct StripCfg {
   static constexpr int S = TS / SR;         // strips per tile
@@ -126,10 +126,21 @@ struct StripCfg {
   static_assert(TS % SR == 0 && PX <= 64, "strip shape");
 };
 
+// Aux channels' part of a strip's shared memory (empty without them).
+template <int SLOTS, int PX, bool AUX>
+struct AuxSmem {
+  float2 aux[SLOTS];           // forward: (t_min, t_max); backward: (aux_s, d a[tet] weight T_prev alpha)
+  float caux[kAuxShared * PX];  // forward: the pixels' first custom channels
+  uint32_t bent[kBatch];       // the batch's entries
+};
+template <int SLOTS, int PX>
+struct AuxSmem<SLOTS, PX, false> {};
+
 template <int TS, int SR, bool AUX>
-struct __align__(16) StripSmem {
+struct __align__(16) StripSmem : AuxSmem<StripCfg<TS, SR>::SLOTS, StripCfg<TS, SR>::PX, AUX> {
   using Cfg = StripCfg<TS, SR>;
-  float4 rec[kBatch][6];        // render records: nrm[4], cb, gm
+  __align__(16) float4 rec[kBatch][6];  // render records: nrm[4], cb, gm
+  float4 v0[kBatch];            // adjoint: the tets' first vertices
   // per item slot (a run's items are consecutive).  Forward: (premultiplied rgb, od).  Adjoint
   // and error: .ex = (od, dl.c) -> (t_prev, d_od_state), .tt = (t_min, t_max)
   union {
@@ -140,17 +151,12 @@ struct __align__(16) StripSmem {
     } a;
   };
   __align__(16) float red[32][kRedCols];  // per-lane moment rows of phase 2
-  // forward: (t_min, t_max); backward: (aux_s, d a[tet] weight T_prev alpha)
-  float2 aux[AUX ? Cfg::SLOTS : 2];
-  float caux[AUX ? kAuxShared * Cfg::PX : 4];  // forward: the pixels' first custom channels
   uint16_t pk[Cfg::SLOTS];      // pack_item
   float4 pdir[Cfg::PX];         // pixel ray direction; w: the pixel's dL/dR (adjoint)
   float2 pdl[Cfg::PX];          // the pixel's dL/dG, dL/dB (adjoint); pixel and SSIM error (error mode)
   uint32_t qw[2 * kBatch];      // gathered pairs waiting for a batch: span word
   uint32_t qv[2 * kBatch];      //   and entry
-  uint32_t bent[AUX ? kBatch : 1];  // the batch's entries
   __align__(8) int16_t rowbase[kBatch][4];  // per (tet, row), one 8-byte store per tet: i0 with i0 + column = run * R + index in run
-  uint16_t piece[36];           // combine: first row | tet slot << 8 of each piece, then the end
 };
 
 __device__ __forceinline__ float4 rec_vertex(const TetRec& r, int i) {
@@ -470,7 +476,8 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
         const uint32_t* sp = (fwd ? a.spans_fwd : a.spans_adj) + (strip * (uint32_t)SR / 4u) * a.span_stride;
         wn = __ldg(sp + pos);
         vn = __ldg(a.pair_val + pos);
-        if (SR == 2) wn = ((wn >> (16u * (strip & 1u))) & 0xFFFFu) | (kEmptySpans << 16);
+        // the strip's rows of the word
+        if (SR < 4) wn = ((wn >> (8u * SR * (strip % (4u / SR)))) & (0xFFFFFFFFu >> (32 - 8 * SR))) | (kEmptySpans << (8 * SR & 31));
       }
     };
     auto start_list = [&](bool fwd) {
@@ -511,7 +518,7 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
         s.qw[lane] = w2;
         s.qv[lane] = v2;
       }
-      if (AUX) s.bent[lane] = bv;
+      if constexpr (AUX) s.bent[lane] = bv;
       // records (the warp has read the previous batch's): six 16-byte pieces each,
       // consecutive lanes on consecutive pieces.  Asynchronous copies of a warp are
       // one instruction for 32 pieces, where a bulk copy per record issues alone.
@@ -521,6 +528,7 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
         const uint32_t entry = __shfl_sync(0xffffffffu, bv, k);
         if (k < nb) async_copy16(&s.rec[0][0] + c, reinterpret_cast<const float4*>(a.vis_view + entry) + (c - 6 * k));
       }
+      if (!fwd && lane < nb) async_copy16(&s.v0[lane], &a.rec[bv / (uint32_t)a.n_views].a);
       // pixels
       uint32_t width;
       bcum = span_prefix(bw, width, bcnt);
@@ -654,14 +662,14 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
             s.pk[slot] = (uint16_t)out_p;
           } else if (fwd) {
             s.item[slot] = out;
-            if (AUX) {
+            if constexpr (AUX) {
               s.aux[slot] = out_t;
               s.pk[slot] = (uint16_t)out_p;
             }
           } else {
             const float2 dgb = s.pdl[p];
             float dlc = d.w * out.x + dgb.x * out.y + dgb.y * out.z;
-            if (AUX && MODE == kModeBackward) {
+            if constexpr (AUX && MODE == kModeBackward) {
               // custom aux channels (aux += T alpha a[tet], rasterize_compute.wgsl:458-462)
               // continue the transmittance chain like a colour alpha a[tet]:
               // aux_s = sum_ai dl_aux[pixel][ai] a[tet][ai]
@@ -703,19 +711,19 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
       static_assert(kMom == 24, "six lanes of four columns");
       const int n_rows = min(32, n_runs - base);
       const unsigned cuts = (heads | 0x01010101u) & (0xffffffffu >> (32 - n_rows));
-      if ((cuts >> lane) & 1u) s.piece[__popc(cuts & (lanes_le >> 1))] = (uint16_t)(lane | (rk << 8));
       const int n_pieces = __popc(cuts);
-      if (lane == 0) s.piece[n_pieces] = (uint16_t)n_rows;
+      // piece i's first row and tet slot, in a padding column of row i
+      if ((cuts >> lane) & 1u) s.red[__popc(cuts & (lanes_le >> 1))][kMom] = __int_as_float(lane | (rk << 8));
       __syncwarp();
       const int sub = lane / 6, col = 4 * (lane - 6 * sub);
       for (int i0 = 0; i0 < n_pieces; i0 += 5) {
         const int i = i0 + sub;
         const bool on = lane < 30 && i < n_pieces;
-        const uint32_t pc = on ? s.piece[i] : 0u;
-        const uint32_t entry = __shfl_sync(0xffffffffu, bv, (int)(pc >> 8));
+        const int pc = on ? __float_as_int(s.red[i][kMom]) : 0;
+        const uint32_t entry = __shfl_sync(0xffffffffu, bv, pc >> 8);
         if (on) {
-          const int r1 = (int)(s.piece[i + 1] & 255u);
-          int r = (int)(pc & 255u);
+          const int r1 = i + 1 < n_pieces ? __float_as_int(s.red[i + 1][kMom]) & 255 : n_rows;
+          int r = pc & 255;
           float4 sum = *reinterpret_cast<const float4*>(&s.red[r][col]);
           for (++r; r < r1; ++r) {
             const float4 v = *reinterpret_cast<const float4*>(&s.red[r][col]);
@@ -760,7 +768,7 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
       float nd[AUX ? NPX : 1][4], en[AUX ? NPX : 1][4];
 #pragma unroll
       for (int q = 0; q < NPX; ++q) {
-        if (AUX) {
+        if constexpr (AUX) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) nd[q][i] = en[q][i] = 0.0f;
           // custom aux channels (rasterize_compute.wgsl:458-462): the first accumulate
@@ -805,7 +813,7 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
               logT[q] -= on ? c.w : 0.0f;
               if (logT[q] < -13.8f) m[q] = 0u;  // saturated: the rest is skipped
               any |= m[q];
-              if (AUX) {
+              if constexpr (AUX) {
                 if (!on) continue;
                 const float2 c2 = s.aux[slot];
                 const float t_min = c2.x, t_max = c2.y;
@@ -856,10 +864,11 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
         if (valid[q] && (MODE == kModeForward || a.rgba != nullptr)) {
           const float A = 1.0f - safe_exp(logT[q]);
           reinterpret_cast<float4*>(a.rgba)[pix[q]] = make_float4(Cr[q], Cg[q], Cb[q], A);
-          if (AUX && a.aux && a.aux_dim == 0) {
+          if constexpr (AUX) {
+          if (a.aux_dim == 0) {
             reinterpret_cast<float4*>(a.aux)[2 * pix[q]] = make_float4(nd[q][0], nd[q][1], nd[q][2], nd[q][3]);
             reinterpret_cast<float4*>(a.aux)[2 * pix[q] + 1] = make_float4(en[q][0], en[q][1], en[q][2], en[q][3]);
-          } else if (AUX && a.aux) {  // [normal.xyz, depth, entropy.4, custom...] (:486-500)
+          } else {  // [normal.xyz, depth, entropy.4, custom...] (:486-500)
             float* o = a.aux + pix[q] * (size_t)(8 + a.aux_dim);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -867,6 +876,7 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
               o[4 + i] = en[q][i];
             }
             for (int ai = 0; ai < min(a.aux_dim, kAuxShared); ++ai) o[8 + ai] = s.caux[ai * PX + 32 * q + lane];
+          }
           }
         }
       }
@@ -1042,9 +1052,10 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
           // unflipped normal n, hit h = cam + d t and s = dT / (n.d), the item
           // adds s (a-h) x (c-a) to vertex b, s (a-h) x (a-b) to c and
           // s ((a-h) x (b-c) + n) to a (backward_tiled_compute.wgsl:506-533).
-          // Since a - h = (a - cam) - t d, the sum over a tet's items needs only
-          // S = sum s and P = sum s t d per face; the vertex gradients are
-          // rebuilt from them once per tet and view (grad_finalize_kernel).  The
+          // The sum over a tet's items needs only S = sum s and P = sum s (h - v0) per
+          // face (v0: the tet's first vertex, so that the differences are taken item
+          // by item and nothing large cancels in the sums, whatever their order);
+          // grad_finalize_kernel rebuilds the vertex gradients from them.  The
           // face sums live in the lane's row of the warp buffer, so the item's
           // entry / exit face is an address (one 16-byte read and write), not a
           // 16-way select; the other 8 sums stay in registers.
@@ -1057,6 +1068,8 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
           if (rlen > 0) {
             const float4 cb = s.rec[rk][4], gg = s.rec[rk][5];
             const uint32_t flips = __float_as_uint(gg.w);
+            const float4 v0 = s.v0[rk];
+            const float rx = V.cam[0] - v0.x, ry = V.cam[1] - v0.y, rz = V.cam[2] - v0.z;
             int slot = lane * R;
 #pragma unroll 1
             for (int j = 0; j < rlen; ++j, ++slot) {
@@ -1086,7 +1099,7 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
               const float d_od_int = dcpr * (I.cer * dw0 + I.csr * dw1) + dcpg * (I.ceg * dw0 + I.csg * dw1) +
                                      dcpb * (I.ceb * dw0 + I.csb * dw1);
               float d_od_aux = 0.0f;
-              if (AUX && MODE == kModeBackward) {
+              if constexpr (AUX && MODE == kModeBackward) {
                 // the aux channels' own terms: d od += T_prev alpha_t aux_s (d alpha / d od =
                 // alpha_t); d a[tet][ai] += dl_aux[pixel][ai] T_prev alpha, below
                 d_od_aux = t_prev * I.alpha_t * s.aux[slot].x;
@@ -1103,7 +1116,9 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
                           deb = I.ceb > 0.f ? dcpb * I.w0 : 0.f;
               const float dbr = dsr + der, dbg = dsg + deg, dbb = dsb + deb;
               const float ss = dsr + dsg + dsb, se = der + deg + deb;
-              const float d_dcdt = ss * t_min + se * t_max;
+              // hits relative to v0
+              const float3 hi = make_float3(rx + d.x * t_min, ry + d.y * t_min, rz + d.z * t_min);
+              const float3 ho = make_float3(rx + d.x * t_max, ry + d.y * t_max, rz + d.z * t_max);
               d_tmin += ss * dcdt;
               d_tmax += se * dcdt;
               acc[0] += clipf(d_od_raw * I.dist, kMinVal, kMaxVal);
@@ -1112,28 +1127,28 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
               acc[2] += dbg;
               acc[3] += dbb;
               acc[4] += dbr + dbg + dbb;
-              acc[5] += d.x * d_dcdt;
-              acc[6] += d.y * d_dcdt;
-              acc[7] += d.z * d_dcdt;
+              acc[5] += ss * hi.x + se * ho.x;
+              acc[6] += ss * hi.y + se * ho.y;
+              acc[7] += ss * hi.z + se * ho.z;
 #pragma unroll
               for (int side = 0; side < 2; ++side) {
                 const int f = side == 0 ? fmin : fmax;
                 const float dt = side == 0 ? d_tmin : d_tmax;
-                const float tt = side == 0 ? t_min : t_max;
+                const float3 h = side == 0 ? hi : ho;
                 const float4 nf = s.rec[rk][f];
                 const float den = (((flips >> f) & 1u) ? -1.0f : 1.0f) * (nf.x * d.x + nf.y * d.y + nf.z * d.z);
                 const float inv_den = fabsf(den) < kTiny ? 1.0f / kTiny : clipf(rcp_fast(den), kMinVal, kMaxVal);
-                const float sv = dt * inv_den, st_ = sv * tt;
+                const float sv = dt * inv_den;
                 float4 v = fac[f];
                 v.x += sv;
-                v.y += st_ * d.x;
-                v.z += st_ * d.y;
-                v.w += st_ * d.z;
+                v.y += sv * h.x;
+                v.z += sv * h.y;
+                v.w += sv * h.z;
                 fac[f] = v;
               }
             }
           }
-          if (AUX && MODE == kModeBackward && rlen > 0) {
+          if constexpr (AUX && MODE == kModeBackward) {
             // the run's aux data gradient, four channels at a time
             float* dst = a.d_aux + (size_t)(rentry / (uint32_t)a.n_views) * a.aux_dim;
             for (int a0 = 0; a0 < a.aux_dim; a0 += 4) {
@@ -1281,7 +1296,6 @@ __global__ void __launch_bounds__(256) pair_spans_kernel(PairSpanArgs a) {
 struct GradFinalizeArgs {
   int M;
   int n_views;
-  const ViewParams* views;
   const TetRec* rec;
   const uint32_t* vis_cnt;  // [M * n_views] tiles touched by the entry
   const float* mom;         // [M * n_views][kMom]
@@ -1304,7 +1318,6 @@ __global__ void __launch_bounds__(128) grad_finalize_kernel(GradFinalizeArgs a) 
     const float4* m4 = reinterpret_cast<const float4*>(a.mom + j * kMom);
     const float4 fs4[4] = {m4[0], m4[1], m4[2], m4[3]};
     const float4 dc = m4[4], sd = m4[5];
-    const float camx = a.views[v].cam[0], camy = a.views[v].cam[1], camz = a.views[v].cam[2];
     const bool inner = dc.x != 0.f || dc.y != 0.f || dc.z != 0.f || dc.w != 0.f || sd.x != 0.f || sd.y != 0.f ||
                        sd.z != 0.f || sd.w != 0.f;
     float dv[12];
@@ -1323,8 +1336,8 @@ __global__ void __launch_bounds__(128) grad_finalize_kernel(GradFinalizeArgs a) 
         // the unflipped normal cross(c - a, b - a), rounded as the record's
         const float nx = fs(fm(e1z, e2y), fm(e1y, e2z)), ny = fs(fm(e1x, e2z), fm(e1z, e2x)),
                     nz = fs(fm(e1y, e2x), fm(e1x, e2y));
-        // w = (a - cam) S - P
-        const float wx = (va.x - camx) * S - Px, wy = (va.y - camy) * S - Py, wz = (va.z - camz) * S - Pz;
+        // w = sum s (a - h) = (a - v0) S - P
+        const float wx = (va.x - r.a.x) * S - Px, wy = (va.y - r.a.y) * S - Py, wz = (va.z - r.a.z) * S - Pz;
         const float bx = wy * e1z - wz * e1y, by = wz * e1x - wx * e1z, bz = wx * e1y - wy * e1x;
         const float cx = wy * e2z - wz * e2y, cy = wz * e2x - wx * e2z, cz = wx * e2y - wy * e2x;
         dv[3 * ia] += nx * S - bx - cx; dv[3 * ia + 1] += ny * S - by - cy; dv[3 * ia + 2] += nz * S - bz - cz;
@@ -1339,9 +1352,9 @@ __global__ void __launch_bounds__(128) grad_finalize_kernel(GradFinalizeArgs a) 
     if (!a.sh) {
       o[1] += dc.y; o[2] += dc.z; o[3] += dc.w;
     }
-    o[4] += clipf((camx - r.a.x) * sb + sd.y, kMinVal, kMaxVal);
-    o[5] += clipf((camy - r.a.y) * sb + sd.z, kMinVal, kMaxVal);
-    o[6] += clipf((camz - r.a.z) * sb + sd.w, kMinVal, kMaxVal);
+    o[4] += clipf(sd.y, kMinVal, kMaxVal);
+    o[5] += clipf(sd.z, kMinVal, kMaxVal);
+    o[6] += clipf(sd.w, kMinVal, kMaxVal);
     dv[0] -= r.b.w * sb; dv[1] -= r.c.w * sb; dv[2] -= r.d.w * sb;
 #pragma unroll
     for (int q = 0; q < 12; ++q) o[7 + q] += clipf(dv[q], kMinVal, kMaxVal);
