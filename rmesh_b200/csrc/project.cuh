@@ -97,14 +97,54 @@ __device__ __forceinline__ bool tile_row_span(const float px[4], const float py[
   tx1 = min(max(tx1, tb.min_x), tb.max_x);
   return true;
 }
+// Crossings of the tet's edges with the row boundary y = row * TS.
+__device__ __forceinline__ void boundary_cross(const float px[4], const float py[4], float ytest, float& xl, float& xr) {
+  const int ei[6] = {0, 0, 0, 1, 1, 2};
+  const int ej[6] = {1, 2, 3, 2, 3, 3};
+  xl = 1e10f;
+  xr = -1e10f;
+#pragma unroll
+  for (int e = 0; e < 6; ++e) {
+    const float yi = py[ei[e]], yj = py[ej[e]], xi = px[ei[e]], xj = px[ej[e]];
+    if ((yi <= ytest && yj > ytest) || (yj <= ytest && yi > ytest)) {
+      const float t = fdv(fs(ytest, yi), fs(yj, yi));
+      const float x = fa(xi, fm(t, fs(xj, xi)));
+      xl = fminf(xl, x);
+      xr = fmaxf(xr, x);
+    }
+  }
+}
+// f(ty, tx0, tx1) for every tile row with a non-empty clamped span: tile_row_span
+// of each row, walked downwards so that a boundary's crossings (a third of them
+// exact divisions) are taken once for the two rows that share it.
 template <class F>
 __device__ __forceinline__ void scanline_tiles(const float px[4], const float py[4], float W, float H, uint32_t TS,
                                                F&& f) {
   TileBox tb;
   if (!tile_range(px, py, W, H, TS, tb)) return;
+  const float T = (float)TS;
+  float al, ar;
+  boundary_cross(px, py, fm((float)tb.min_y, T), al, ar);
   for (uint32_t ty = tb.min_y; ty <= tb.max_y; ++ty) {
-    uint32_t tx0, tx1;
-    if (tile_row_span(px, py, TS, tb, ty, tx0, tx1)) f(ty, tx0, tx1);
+    const float band_lo = fm((float)ty, T), band_hi = fm((float)(ty + 1u), T);
+    float bl, br;
+    boundary_cross(px, py, band_hi, bl, br);
+    float xl = fminf(al, bl), xr = fmaxf(ar, br);
+    al = bl;
+    ar = br;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      if (py[v] >= band_lo && py[v] <= band_hi) {
+        xl = fminf(xl, px[v]);
+        xr = fmaxf(xr, px[v]);
+      }
+    }
+    if (!(xl <= xr)) continue;
+    uint32_t tx0 = __float2uint_rz(fmaxf(floorf(fdv(xl, T)), 0.0f));
+    uint32_t tx1 = __float2uint_rz(fmaxf(floorf(fdv(xr, T)), 0.0f));
+    tx0 = min(max(tx0, tb.min_x), tb.max_x);
+    tx1 = min(max(tx1, tb.min_x), tb.max_x);
+    f(ty, tx0, tx1);
   }
 }
 
