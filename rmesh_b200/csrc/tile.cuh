@@ -65,9 +65,11 @@ __device__ __forceinline__ uint8_t pack_span(short2 sp) {
 constexpr int kMom = 24;
 // error statistics per tet: 11 sums and a maximum
 constexpr int kErrMom = 12;
-// per-lane row of the warp's reduction buffer: 24 columns, padded so that a
-// column of 16-byte accesses hits distinct banks (112-byte stride)
-constexpr int kRedCols = 28;
+// per-lane rows of the warp's reduction buffers, with strides that spread a column
+// of 16-byte accesses over all banks: the 16 face sums (column 16 free), and the
+// other 8 sums (in the item area, once the round's items have been read)
+constexpr int kRedCols = 20;
+constexpr int kSumCols = 12;
 constexpr int kStripWarps = 4;  // warps (independent strips) per CTA
 
 constexpr int kAuxShared = 8;   // custom aux channels accumulated in shared memory
@@ -119,11 +121,13 @@ struct StripCfg {
   static constexpr int S = TS / SR;         // strips per tile
   static constexpr int PX = TS * SR;        // pixels per strip (at most 64)
   static constexpr int NPX = (PX + 31) / 32;  // pixels per lane
-  // items per run, sized for shared memory; run lengths are odd, so that lanes
-  // at the same place of their runs hit distinct banks
-  static constexpr int RMAX = TS == 16 ? 7 : 9;
+  // items per run, as many as leave room for five CTAs per SM (four for 16-pixel
+  // tiles); run lengths are odd, so that lanes at the same place of their runs
+  // hit distinct banks
+  static constexpr int RMAX = SR == 4 ? 5 : 7;
   static constexpr int SLOTS = 32 * RMAX;
   static_assert(TS % SR == 0 && PX <= 64, "strip shape");
+  static_assert(RMAX % 2 == 1 && 16 * SLOTS >= 4 * 32 * kSumCols, "run length, room for the sums");
 };
 
 // Aux channels' part of a strip's shared memory (empty without them).
@@ -156,7 +160,7 @@ struct __align__(16) StripSmem : AuxSmem<StripCfg<TS, SR>::SLOTS, StripCfg<TS, S
   float2 pdl[Cfg::PX];          // the pixel's dL/dG, dL/dB (adjoint); pixel and SSIM error (error mode)
   uint32_t qw[2 * kBatch];      // gathered pairs waiting for a batch: span word
   uint32_t qv[2 * kBatch];      //   and entry
-  __align__(8) int16_t rowbase[kBatch][4];  // per (tet, row), one 8-byte store per tet: i0 with i0 + column = run * R + index in run
+  __align__(8) int16_t rowbase[kBatch][SR];  // per (tet, row): i0 with i0 + column = run * R + index in run
 };
 
 __device__ __forceinline__ float4 rec_vertex(const TetRec& r, int i) {
@@ -385,9 +389,20 @@ __device__ __forceinline__ uint32_t span_prefix(uint32_t w, uint32_t& width, int
   return incl - width;
 }
 
-// strip_kernel: bound by instruction issue.
+// Bound by instruction issue and, at four to five warps per scheduler, by the
+// latency between dependent instructions: one 801x603 step (19.8 M crossings,
+// 0.57 M pairs) issues 0.74 instructions per cycle and scheduler, DRAM 1 % busy.
+// Its tile-kernel time, before strips and after each step: 1.233 ms; strips with
+// the branch-free division 1.100; branch-free compositing 0.982; combine in
+// pieces, warp-wide copies 0.824; two-row strips 0.784; five CTAs per SM 0.753
+// (96 registers, a few spills outside the item loops; shorter runs).  The
+// adjoint alone keeps four CTAs: its launches are one view's, where the longest
+// strip counts (512x512, 66 k tets, forward + adjoint: 0.418 against 0.444 ms).
+// Packed two-float arithmetic (FFMA2) cut the instructions by 2 % and the time
+// by nothing.
 template <int TS, int SR, int MODE, bool AUX>
-__global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(TileArgs a) {
+__global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : (TS == 16 || MODE == kModeBackward ? 4 : 5))
+    strip_kernel(TileArgs a) {
   using Cfg = StripCfg<TS, SR>;
   constexpr int S = Cfg::S, PX = Cfg::PX, NPX = Cfg::NPX, RMAX = Cfg::RMAX;
   using PMask = typename PixMask<(PX > 32)>::T;
@@ -541,11 +556,11 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
       // run length: the cheapest of a few, a round costing about its longest
       // run plus one item's work for the set-up and the combine
       const int cmax = __reduce_max_sync(0xffffffffu, bcnt);
-      constexpr int kCand[4] = {RMAX, 7, 5, 3};
+      constexpr int kCand[3] = {RMAX, RMAX > 5 ? 5 : 3, 3};
       int best = 0x7fffffff;
       uint32_t rmul = 0u;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < (RMAX > 5 ? 3 : 2); ++i) {
         const int total = __reduce_add_sync(0xffffffffu, (bcnt + kCand[i] - 1) / kCand[i]);
         const int cost = ((total + 31) >> 5) * (min(kCand[i], cmax) + 1);
         if (cost < best) {
@@ -565,12 +580,12 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
       n_runs = __shfl_sync(0xffffffffu, x, 31);
       {
         const int i0 = brun * R;
-        int b[4];
+        int b[SR];
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
+        for (int r = 0; r < SR; ++r)
           b[r] = i0 + (int)((bcum >> (8 * r)) & 255u) - (int)((bw >> (8 * r + 4)) & 15u);
-        *reinterpret_cast<uint2*>(&s.rowbase[lane][0]) =
-            make_uint2(((uint32_t)b[0] & 0xFFFFu) | ((uint32_t)b[1] << 16), ((uint32_t)b[2] & 0xFFFFu) | ((uint32_t)b[3] << 16));
+#pragma unroll
+        for (int r = 0; r < SR; ++r) s.rowbase[lane][r] = (int16_t)b[r];
       }
 #pragma unroll
       for (int q = 0; q < NPX; ++q) tmask[q] = warp_transpose_bits((uint32_t)(bmask >> (q ? 32 : 0)), lane);
@@ -691,7 +706,7 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
     // the round's last run may continue in the next round: its item at this pixel
     // is looked up once.
     auto take_tets = [&](int q, int base, bool on) -> uint32_t {
-      const int row = (32 * q + lane) / TS & 3, col = (32 * q + lane) % TS;
+      const int row = (32 * q + lane) / TS & (SR - 1), col = (32 * q + lane) % TS;
       uint32_t m = on ? tmask[q] & ((2u << rklast) - 1u) : 0u;
       if ((m >> rklast) & 1u) {
         if ((int)s.rowbase[rklast][row] + col >= (base + 32) * R) m ^= 1u << rklast;
@@ -701,7 +716,7 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
     };
     // slot of (tet k, this lane's pixel q) in the round that starts at run `base`
     auto slot_of = [&](int k, int q, int base) -> int {
-      const int row = (32 * q + lane) / TS & 3, col = (32 * q + lane) % TS;
+      const int row = (32 * q + lane) / TS & (SR - 1), col = (32 * q + lane) % TS;
       return (int)s.rowbase[k][row] + (col - base * R);
     };
     // adds the lanes' rows (one per run) to `dst` per tet.  The rows are cut into
@@ -713,20 +728,22 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
       const unsigned cuts = (heads | 0x01010101u) & (0xffffffffu >> (32 - n_rows));
       const int n_pieces = __popc(cuts);
       // piece i's first row and tet slot, in a padding column of row i
-      if ((cuts >> lane) & 1u) s.red[__popc(cuts & (lanes_le >> 1))][kMom] = __int_as_float(lane | (rk << 8));
+      if ((cuts >> lane) & 1u) s.red[__popc(cuts & (lanes_le >> 1))][16] = __int_as_float(lane | (rk << 8));
       __syncwarp();
       const int sub = lane / 6, col = 4 * (lane - 6 * sub);
+      const float* src = col < 16 ? &s.red[0][col] : reinterpret_cast<const float*>(&s.item[0]) + (col - 16);
+      const int stride = col < 16 ? kRedCols : kSumCols;
       for (int i0 = 0; i0 < n_pieces; i0 += 5) {
         const int i = i0 + sub;
         const bool on = lane < 30 && i < n_pieces;
-        const int pc = on ? __float_as_int(s.red[i][kMom]) : 0;
+        const int pc = on ? __float_as_int(s.red[i][16]) : 0;
         const uint32_t entry = __shfl_sync(0xffffffffu, bv, pc >> 8);
         if (on) {
-          const int r1 = i + 1 < n_pieces ? __float_as_int(s.red[i + 1][kMom]) & 255 : n_rows;
+          const int r1 = i + 1 < n_pieces ? __float_as_int(s.red[i + 1][16]) & 255 : n_rows;
           int r = pc & 255;
-          float4 sum = *reinterpret_cast<const float4*>(&s.red[r][col]);
+          float4 sum = *reinterpret_cast<const float4*>(src + r * stride);
           for (++r; r < r1; ++r) {
-            const float4 v = *reinterpret_cast<const float4*>(&s.red[r][col]);
+            const float4 v = *reinterpret_cast<const float4*>(src + r * stride);
             sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
           }
           if (sum.x != 0.0f || sum.y != 0.0f || sum.z != 0.0f || sum.w != 0.0f)
@@ -1165,8 +1182,12 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : 4) strip_kernel(Ti
                 if (a0 + i < a.aux_dim && sum[i] != 0.0f) atomicAdd(dst + a0 + i, sum[i]);
             }
           }
-          fac[4] = make_float4(acc[0], acc[1], acc[2], acc[3]);
-          fac[5] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+          __syncwarp();  // every lane has read its items
+          {
+            float4* sums = reinterpret_cast<float4*>(&s.item[0]) + (kSumCols / 4) * lane;
+            sums[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+            sums[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+          }
           __syncwarp();
           combine(base, a.mom);
           __syncwarp();
