@@ -522,8 +522,9 @@ int run_records(RmeshCtx* c, bool capturing) {
 }
 
 // project -> tet sort -> emit -> pair sort -> ranges for n_views views at views_dev
+// (adjoint: the run's lists will also be walked by the adjoint)
 int run_bin(RmeshCtx* c, const ViewParams* views_dev, int n_views, uint32_t total_tiles, Counters* cnt,
-            bool capturing, const std::vector<TileGroup>& groups) {
+            bool capturing, const std::vector<TileGroup>& groups, bool adjoint = true) {
   const uint64_t items = (uint64_t)n_views * (uint64_t)c->M;
   // chained scans over blocks of kCompactItems items (key compaction) and
   // sorted entries (pair offsets)
@@ -613,10 +614,6 @@ int run_bin(RmeshCtx* c, const ViewParams* views_dev, int n_views, uint32_t tota
   {
     StageScope sc(c, kStRanges, capturing);
     CK(cudaMemsetAsync(c->ranges.p, 0, (size_t)total_tiles * 8, c->stream));
-    const int blocks = (int)std::min<uint64_t>((c->cap_pairs + 255) / 256, (uint64_t)c->num_sms * 16);
-    ranges_kernel<<<std::max(1, blocks), 256, 0, c->stream>>>(c->sorted_pair_key, &cnt->n_pairs, c->cap_pairs,
-                                                               c->ranges.as<uint2>(), views_dev, n_views, cnt);
-    CKL();
     PairSpanArgs sa;
     sa.views = views_dev;
     sa.n_views = n_views;
@@ -626,8 +623,10 @@ int run_bin(RmeshCtx* c, const ViewParams* views_dev, int n_views, uint32_t tota
     sa.cap = c->cap_pairs;
     sa.vis_view = c->vis_view.as<TetView>();
     sa.spans_fwd = c->spans_fwd.as<uint32_t>();
-    sa.spans_adj = c->spans_adj.as<uint32_t>();
+    sa.spans_adj = adjoint ? c->spans_adj.as<uint32_t>() : nullptr;
     sa.stride = c->cap_pairs;
+    sa.ranges = c->ranges.as<uint2>();
+    sa.counters = cnt;
     const int sblocks = (int)std::min<uint64_t>((c->cap_pairs + 255) / 256, (uint64_t)c->num_sms * 8);
     pair_spans_kernel<<<std::max(1, sblocks), 256, 0, c->stream>>>(sa);
     CKL();
@@ -1441,7 +1440,7 @@ int rmesh_forward_views(RmeshCtx* c, const RmeshCamera* cams, int32_t n_views, f
     CK(cudaMemsetAsync(cnt, 0, sizeof(Counters), c->stream));
     CKR(run_records(c, false));
     ViewParams* vd = c->views_d.as<ViewParams>();
-    CKR(run_bin(c, vd, n_views, total_tiles, cnt, false, pl.groups));
+    CKR(run_bin(c, vd, n_views, total_tiles, cnt, false, pl.groups, false));
     {
       StageScope sc(c, kStComposite, false);
       TileArgs ta = base_tile_args(c, vd, n_views, total_tiles, cnt);

@@ -319,32 +319,6 @@ __global__ void __launch_bounds__(kOrderThreads) tile_order_stable_kernel(const 
   }
 }
 
-// Per-tile [start, end) over the sorted pair keys.  Restates
-// tile_ranges_compute.wgsl:10-45 per view: the end of a view's last non-empty
-// tile is only written when the view had no sentinel slots (in the reference
-// the sentinels follow that tile and the idx == count-1 rule never fires for
-// it, leaving end = 0 from the clear).  ranges must be zeroed beforehand.
-__global__ void __launch_bounds__(256) ranges_kernel(const uint32_t* __restrict__ keys,
-                                                     const unsigned long long* n_ptr, unsigned long long cap,
-                                                     uint2* __restrict__ ranges,
-                                                     const ViewParams* views, int n_views,
-                                                     const Counters* counters) {
-  const unsigned long long n = *n_ptr < cap ? *n_ptr : cap;
-  for (unsigned long long idx = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; idx < n;
-       idx += (unsigned long long)gridDim.x * blockDim.x) {
-    const uint32_t key = keys[idx];
-    if (key == kSentinel) continue;
-    const uint32_t prev = idx > 0 ? keys[idx - 1] : kSentinel;
-    const uint32_t next = idx + 1 < n ? keys[idx + 1] : kSentinel;
-    if (idx == 0 || key != prev) ranges[key].x = (uint32_t)idx;
-    if (next != key) {
-      const int v = view_of_tile(views, n_views, key);
-      const bool last_of_view = (next == kSentinel) || view_of_tile(views, n_views, next) != v;
-      if (!(last_of_view && counters->shortfall[v])) ranges[key].y = (uint32_t)(idx + 1);
-    }
-  }
-}
-
 // Debug view of the sorted pairs: the pair payload is the item index
 // tet * n_views + view; map it back to the tet id (sentinel slots keep the
 // reference's 0).

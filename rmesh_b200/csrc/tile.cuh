@@ -295,48 +295,48 @@ __device__ __forceinline__ short2 span_of_cols(float xl, float xr, int valid_col
   }
   return sp;
 }
-// sx, sy: the four vertices sorted by y.  An edge crosses the row's centre
-// line yc when its lower end is <= yc < its upper end, so with b vertices at
-// or below yc the crossing edges are exactly the pairs (i, j) of sorted ranks
-// i < b <= j: three edges for b = 1 or 3, four for b = 2, none otherwise.
-__device__ __forceinline__ void row_spans(const float sx[4], const float sy[4], int row, int valid_cols, uint8_t& fwd,
-                                          uint8_t& adj) {
+// One pair's set-up: the four vertices sorted by y and the slopes dx/dy of the
+// edges between sorted ranks (an edge without height crosses no centre line, so
+// its slope is never used).
+struct SpanSetup {
+  float x[4], y[4];
+  float m01, m02, m03, m12, m13, m23;
+  int first_row;   // row of the warp's task t of this pair: first_row + t
+  int valid_cols;  // columns of the tile inside the image
+};
+// An edge crosses the row's centre line yc when its lower end is <= yc < its
+// upper end, so with b vertices at or below yc the crossing edges are exactly
+// the pairs (i, j) of sorted ranks i < b <= j: three edges for b = 1 or 3, four
+// for b = 2, none otherwise.  The adjoint's span comes out empty without
+// crossings; its reach (some edge crosses yc) implies the forward's.
+__device__ __forceinline__ void row_spans(const SpanSetup& p, int row, bool adjoint, uint8_t& fwd, uint8_t& adj) {
   fwd = 0xF0u;
   adj = 0xF0u;
   const float yc = fa((float)row, 0.5f);
   const float blo = fs(yc, 0.5f), bhi = fa(yc, 0.5f);
-  // the adjoint's reach (some edge crosses yc) implies the forward's
-  if (!(sy[3] >= blo && sy[0] < bhi)) return;
-  const int nb = (sy[0] <= yc ? 1 : 0) + (sy[1] <= yc ? 1 : 0) + (sy[2] <= yc ? 1 : 0) + (sy[3] <= yc ? 1 : 0);
+  if (!(p.y[3] >= blo && p.y[0] < bhi)) return;
+  const int nb = (p.y[0] <= yc ? 1 : 0) + (p.y[1] <= yc ? 1 : 0) + (p.y[2] <= yc ? 1 : 0) + (p.y[3] <= yc ? 1 : 0);
   float xl = 1e10f, xr = -1e10f;
-  auto cross = [&](float xi, float yi, float xj, float yj) {
-    const float t = __fdividef(yc - yi, yj - yi);
-    const float x = xi + t * (xj - xi);
-    xl = fminf(xl, x);
-    xr = fmaxf(xr, x);
-  };
   if (nb >= 1 && nb <= 3) {
-    cross(sx[0], sy[0], sx[3], sy[3]);  // (0, 3) crosses in every band
+    const float d0 = yc - p.y[0], d1 = yc - p.y[1];
+    const float a = p.x[0] + d0 * p.m03;  // (0, 3) crosses in every band
     // (0, 1) | (0, 2) | (1, 3) for b = 1 | 2 | 3
-    const float ax = nb == 3 ? sx[1] : sx[0], ay = nb == 3 ? sy[1] : sy[0];
-    const float bx = nb == 1 ? sx[1] : (nb == 2 ? sx[2] : sx[3]), by = nb == 1 ? sy[1] : (nb == 2 ? sy[2] : sy[3]);
-    cross(ax, ay, bx, by);
+    const float b = nb == 3 ? p.x[1] + d1 * p.m13 : p.x[0] + d0 * (nb == 1 ? p.m01 : p.m02);
     // (0, 2) | (1, 2) | (2, 3)
-    const float cx = nb == 1 ? sx[0] : (nb == 2 ? sx[1] : sx[2]), cy = nb == 1 ? sy[0] : (nb == 2 ? sy[1] : sy[2]);
-    const float dx = nb == 3 ? sx[3] : sx[2], dy = nb == 3 ? sy[3] : sy[2];
-    cross(cx, cy, dx, dy);
-    if (nb == 2) cross(sx[1], sy[1], sx[3], sy[3]);  // (1, 3)
+    const float c = nb == 1 ? p.x[0] + d0 * p.m02 : (nb == 2 ? p.x[1] + d1 * p.m12 : p.x[2] + (yc - p.y[2]) * p.m23);
+    const float d = nb == 2 ? p.x[1] + d1 * p.m13 : a;  // (1, 3)
+    xl = fminf(fminf(a, b), fminf(c, d));
+    xr = fmaxf(fmaxf(a, b), fmaxf(c, d));
   }
-  adj = pack_span(span_of_cols(xl, xr, valid_cols));  // empty when no edge crosses yc
+  if (adjoint) adj = pack_span(span_of_cols(xl, xr, p.valid_cols));
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    const float vyq = sy[q];
-    if (vyq >= blo && vyq < bhi) {
-      xl = fminf(xl, sx[q]);
-      xr = fmaxf(xr, sx[q]);
+    if (p.y[q] >= blo && p.y[q] < bhi) {
+      xl = fminf(xl, p.x[q]);
+      xr = fmaxf(xr, p.x[q]);
     }
   }
-  fwd = pack_span(span_of_cols(xl, xr, valid_cols));
+  fwd = pack_span(span_of_cols(xl, xr, p.valid_cols));
 }
 
 // pk packs the adjoint's entry (0..4) and exit (0..3) faces and the strip pixel (0..63)
@@ -1202,10 +1202,17 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : (TS == 16 || MODE 
 // row (pack_span, row_spans), four rows per 32-bit word, over the rows its tet
 // reaches; a strip of the tile kernel reads the word of its rows.  Other rows,
 // tets with a vertex behind the camera and sentinel slots get empty spans.  Each
-// warp takes 32 consecutive pairs; lane l sets up pair l, and the warp's (pair,
-// row) tasks are spread over its lanes through a prefix of the row counts, so
-// lanes stay busy whatever the rows per tet.  The rows go to shared memory; the
-// owner lane then stores the pair's words, each word array coalesced.
+// warp takes 32 consecutive pairs; lane l sets up pair l (sorted vertices, edge
+// slopes) in shared memory, and the warp's (pair, row) tasks are spread over its
+// lanes through a prefix of the row counts, so lanes stay busy whatever the rows
+// per tet.  The rows go to shared memory; the owner lane then stores the pair's
+// words, each word array coalesced.
+//
+// The same pass over the keys finds the tiles' [start, end): it restates
+// tile_ranges_compute.wgsl:10-45 per view, where the end of a view's last
+// non-empty tile is only written when the view had no sentinel slots (in the
+// reference the sentinels follow that tile and the idx == count-1 rule never
+// fires for it, leaving end = 0 from the clear).  ranges must be zeroed beforehand.
 struct PairSpanArgs {
   const ViewParams* views;
   int n_views;
@@ -1215,58 +1222,73 @@ struct PairSpanArgs {
   unsigned long long cap;
   const TetView* vis_view;
   uint32_t* spans_fwd;  // word w of pair i at [w * stride + i]
-  uint32_t* spans_adj;
+  uint32_t* spans_adj;  // nullptr: a run without an adjoint
   unsigned long long stride;
+  uint2* ranges;
+  const Counters* counters;
 };
 
 __global__ void __launch_bounds__(256) pair_spans_kernel(PairSpanArgs a) {
   __shared__ __align__(16) uint8_t s_fwd[256][4 * kSpanWords];
   __shared__ __align__(16) uint8_t s_adj[256][4 * kSpanWords];
+  __shared__ __align__(16) SpanSetup s_set[256];
+  static_assert(sizeof(SpanSetup) == 64, "four 16-byte reads");
   const int lane = threadIdx.x & 31, wbase = threadIdx.x & ~31;
   const unsigned long long n = *a.n_ptr < a.cap ? *a.n_ptr : a.cap;
-  const uint4 empty = make_uint4(0xF0F0F0F0u, 0xF0F0F0F0u, 0xF0F0F0F0u, 0xF0F0F0F0u);
+  const bool adjoint = a.spans_adj != nullptr;
+  const uint4 empty = make_uint4(kEmptySpans, kEmptySpans, kEmptySpans, kEmptySpans);
   for (unsigned long long base = (unsigned long long)blockIdx.x * blockDim.x; base < n;
        base += (unsigned long long)gridDim.x * blockDim.x) {
     const unsigned long long p = base + threadIdx.x;
     *reinterpret_cast<uint4*>(s_fwd[threadIdx.x]) = empty;
     *reinterpret_cast<uint4*>(s_adj[threadIdx.x]) = empty;
-    float vpx[4] = {0.f, 0.f, 0.f, 0.f}, vpy[4] = {0.f, 0.f, 0.f, 0.f};
-    int valid_cols = 0, r0 = 0, nrows = 0;
+    SpanSetup st;
+    st.valid_cols = 0;
+    int r0 = 0, nrows = 0;
     int words = kSpanWords;  // words of the pair's tile size
-    if (p < n) {
-      const uint32_t key = a.keys[p];
-      if (key != kSentinel) {
-        const ViewParams& V = a.views[view_of_tile(a.views, a.n_views, key)];
-        const int TS = V.TS;
-        words = (TS + 3) / 4;
-        const uint32_t local = key - V.tile_base;
-        const uint32_t ty = local / (uint32_t)V.tiles_x, tx = local - ty * (uint32_t)V.tiles_x;
-        valid_cols = min(TS, V.W - (int)(tx * (uint32_t)TS));
-        const int valid_rows = min(TS, V.H - (int)(ty * (uint32_t)TS));
-        const TetView* tv = a.vis_view + a.vals[p];
-        if (!((__float_as_uint(__ldg(&tv->gm.w)) >> 4) & 1u)) {
-          const float4 gx4 = __ldg(&tv->px), gy4 = __ldg(&tv->py);
-          const float tile_ox = (float)(tx * (uint32_t)TS), tile_oy = (float)(ty * (uint32_t)TS);
-          vpx[0] = gx4.x - tile_ox; vpx[1] = gx4.y - tile_ox; vpx[2] = gx4.z - tile_ox; vpx[3] = gx4.w - tile_ox;
-          vpy[0] = gy4.x - tile_oy; vpy[1] = gy4.y - tile_oy; vpy[2] = gy4.z - tile_oy; vpy[3] = gy4.w - tile_oy;
-          // the vertices sorted by y (five compare-exchanges), as row_spans takes them
-          auto cx = [&](int i, int j) {
-            if (vpy[j] < vpy[i]) {
-              const float ty = vpy[i], tx = vpx[i];
-              vpy[i] = vpy[j]; vpx[i] = vpx[j];
-              vpy[j] = ty; vpx[j] = tx;
-            }
-          };
-          cx(0, 1); cx(2, 3); cx(0, 2); cx(1, 3); cx(1, 2);
-          // rows r with floor(ylo) <= r <= floor(yhi), clipped to the image: the
-          // only rows the forward's reach rule can accept
-          const float ylo = vpy[0], yhi = vpy[3];
-          const float flo = fmaxf(floorf(ylo), 0.0f);
-          const float fhi = fminf(floorf(yhi), (float)(valid_rows - 1));
-          if (flo <= fhi) {
-            r0 = (int)flo;
-            nrows = (int)fhi - r0 + 1;
+    const uint32_t key = p < n ? a.keys[p] : kSentinel;
+    uint32_t prev = __shfl_up_sync(0xffffffffu, key, 1), next = __shfl_down_sync(0xffffffffu, key, 1);
+    if (key != kSentinel) {
+      if (lane == 0) prev = p > 0 ? a.keys[p - 1] : kSentinel;
+      if (lane == 31) next = p + 1 < n ? a.keys[p + 1] : kSentinel;
+      const int view = view_of_tile(a.views, a.n_views, key);
+      if (key != prev) a.ranges[key].x = (uint32_t)p;
+      if (key != next) {
+        const bool last_of_view = next == kSentinel || view_of_tile(a.views, a.n_views, next) != view;
+        if (!(last_of_view && a.counters->shortfall[view])) a.ranges[key].y = (uint32_t)(p + 1);
+      }
+      const ViewParams& V = a.views[view];
+      const int TS = V.TS;
+      words = (TS + 3) / 4;
+      const uint32_t local = key - V.tile_base;
+      const uint32_t ty = local / (uint32_t)V.tiles_x, tx = local - ty * (uint32_t)V.tiles_x;
+      st.valid_cols = min(TS, V.W - (int)(tx * (uint32_t)TS));
+      const int valid_rows = min(TS, V.H - (int)(ty * (uint32_t)TS));
+      const TetView* tv = a.vis_view + a.vals[p];
+      if (!((__float_as_uint(__ldg(&tv->gm.w)) >> 4) & 1u)) {
+        const float4 gx4 = __ldg(&tv->px), gy4 = __ldg(&tv->py);
+        const float tile_ox = (float)(tx * (uint32_t)TS), tile_oy = (float)(ty * (uint32_t)TS);
+        st.x[0] = gx4.x - tile_ox; st.x[1] = gx4.y - tile_ox; st.x[2] = gx4.z - tile_ox; st.x[3] = gx4.w - tile_ox;
+        st.y[0] = gy4.x - tile_oy; st.y[1] = gy4.y - tile_oy; st.y[2] = gy4.z - tile_oy; st.y[3] = gy4.w - tile_oy;
+        // sorted by y (five compare-exchanges)
+        auto cx = [&](int i, int j) {
+          if (st.y[j] < st.y[i]) {
+            const float ty = st.y[i], tx = st.x[i];
+            st.y[i] = st.y[j]; st.x[i] = st.x[j];
+            st.y[j] = ty; st.x[j] = tx;
           }
+        };
+        cx(0, 1); cx(2, 3); cx(0, 2); cx(1, 3); cx(1, 2);
+        auto slope = [&](int i, int j) { return __fdividef(st.x[j] - st.x[i], st.y[j] - st.y[i]); };
+        st.m01 = slope(0, 1); st.m02 = slope(0, 2); st.m03 = slope(0, 3);
+        st.m12 = slope(1, 2); st.m13 = slope(1, 3); st.m23 = slope(2, 3);
+        // rows r with floor(ylo) <= r <= floor(yhi), clipped to the image: the
+        // only rows the forward's reach rule can accept
+        const float flo = fmaxf(floorf(st.y[0]), 0.0f);
+        const float fhi = fminf(floorf(st.y[3]), (float)(valid_rows - 1));
+        if (flo <= fhi) {
+          r0 = (int)flo;
+          nrows = (int)fhi - r0 + 1;
         }
       }
     }
@@ -1277,25 +1299,22 @@ __global__ void __launch_bounds__(256) pair_spans_kernel(PairSpanArgs a) {
       if (lane >= o) pre += y;
     }
     const int total = __shfl_sync(0xffffffffu, pre, 31);
-    const int first_row = r0 - (pre - nrows);  // row of task t of this lane's pair: first_row + t
-    __syncwarp();  // the records' empty rows are set before any task writes one
+    st.first_row = r0 - (pre - nrows);
+    if (nrows > 0) s_set[threadIdx.x] = st;
+    __syncwarp();  // the set-ups and the records' empty rows, before any task
     for (int t0 = 0; t0 < total; t0 += 32) {  // warp-uniform trip count
       const int t = t0 + lane;
       int k = 0;  // the lane whose pair owns task t: first inclusive prefix > t
 #pragma unroll
-      for (int st = 16; st > 0; st >>= 1) {
-        const int pv = __shfl_sync(0xffffffffu, pre, k + st - 1);
-        if (pv <= t) k += st;
+      for (int st2 = 16; st2 > 0; st2 >>= 1) {
+        const int pv = __shfl_sync(0xffffffffu, pre, k + st2 - 1);
+        if (pv <= t) k += st2;
       }
-      const int row = __shfl_sync(0xffffffffu, first_row, k) + t;
-      const int vc = __shfl_sync(0xffffffffu, valid_cols, k);
-      float qx[4], qy[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        qx[q] = __shfl_sync(0xffffffffu, vpx[q], k);
-        qy[q] = __shfl_sync(0xffffffffu, vpy[q], k);
+      if (t < total) {
+        const SpanSetup q = s_set[wbase + k];
+        const int row = q.first_row + t;
+        row_spans(q, row, adjoint, s_fwd[wbase + k][row], s_adj[wbase + k][row]);
       }
-      if (t < total) row_spans(qx, qy, row, vc, s_fwd[wbase + k][row], s_adj[wbase + k][row]);
     }
     __syncwarp();
     if (p < n) {
@@ -1303,7 +1322,7 @@ __global__ void __launch_bounds__(256) pair_spans_kernel(PairSpanArgs a) {
       const uint32_t* va = reinterpret_cast<const uint32_t*>(s_adj[threadIdx.x]);
       for (int w = 0; w < words; ++w) {
         a.spans_fwd[w * a.stride + p] = vf[w];
-        a.spans_adj[w * a.stride + p] = va[w];
+        if (adjoint) a.spans_adj[w * a.stride + p] = va[w];
       }
     }
     __syncwarp();  // the stores' reads before the next chunk's rows are reset
