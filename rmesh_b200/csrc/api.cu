@@ -114,17 +114,17 @@ struct RmeshCtx {
   DevBuf dl_aux, d_aux;   // backward: [pixels][aux_dim] loss gradient, [M][aux_dim] data gradient
 
   // per-run
-  DevBuf views_d, counters_d, hp_d, sort_state, sort_status, scan_status;
+  DevBuf views_d, counters_d, hp_d, sort_state, sort_status;
+  DevBuf run_state;  // everything a run clears, in one piece (RunState)
   // per (tet, view) item, at tet * n_views + view: tiles touched, projections,
   // tile-kernel record; compacted sort keys and values (item indices)
   DevBuf vis_key, vis_val, vis_cnt, vis_proj, vis_view, vis_key_alt, vis_val_alt, group_off;
   DevBuf vis_color;              // SH colours per entry
   DevBuf mom;                    // adjoint moments per entry (error statistics: per tet)
-  DevBuf pair_key, pair_val, pair_key_alt, pair_val_alt, ranges;
+  DevBuf pair_key, pair_val, pair_key_alt, pair_val_alt;
   DevBuf rgba, aux, dl, gt, out_a, out_b, out_c, out_d;
   DevBuf spans_fwd, spans_adj;  // per sorted pair: span words of its tile rows (forward / adjoint rule)
-  DevBuf tile_order, order_hist;  // longest-first tile order of the run; bucket counts and cursors
-  DevBuf tickets;                 // persistent tile-queue heads, one per launch of a run
+  DevBuf tile_order;  // longest-first tile order of the run
   DevBuf err_in, err_out;  // per-pixel error inputs, per-tet error statistics
   uint64_t cap_pairs = 0;
   uint64_t generation = 0;  // bumped whenever a buffer is reallocated
@@ -137,6 +137,8 @@ struct RmeshCtx {
   // results of the last run
   uint32_t* sorted_pair_key = nullptr;
   uint32_t* sorted_pair_val = nullptr;
+  uint2* ranges = nullptr;      // [start, end) per tile (in run_state)
+  uint32_t* tickets = nullptr;  // persistent strip-queue heads, one per launch of a run (in run_state)
   bool have_forward = false;
   uint32_t last_tiles = 0;
   int last_views = 0;
@@ -355,17 +357,15 @@ struct ViewPlan {
 };
 
 // ---------------------------------------------------------------- sorting
+// hist: zeroed before the call
 template <typename K>
 int radix_sort(RmeshCtx* c, K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt, const void* n_ptr, int n_is_u64,
-               uint64_t cap, int bits, K** out_keys, uint32_t** out_vals, bool capturing) {
+               uint64_t cap, int bits, K** out_keys, uint32_t** out_vals, SortHist* hist) {
   const int passes = std::max(1, (bits + 7) / 8);
   SortState* st = c->sort_state.as<SortState>();
   Counters* cnt = c->counters_d.as<Counters>();
-  CK(cudaMemsetAsync(st->hist, 0, sizeof(st->hist), c->stream));
   const int hist_blocks = (int)std::min<uint64_t>((cap + 255) / 256, (uint64_t)c->num_sms * 8);
-  sort_hist_kernel<K><<<std::max(1, hist_blocks), 256, 0, c->stream>>>(keys, n_ptr, n_is_u64, cap, 0, passes, st);
-  CKL();
-  sort_scan_kernel<<<1, 256, 0, c->stream>>>(passes, st);
+  sort_hist_kernel<K><<<std::max(1, hist_blocks), 256, 0, c->stream>>>(keys, n_ptr, n_is_u64, cap, 0, passes, st, hist);
   CKL();
   constexpr int part = SortCfg<K>::PART;
   const size_t smem = sizeof(K) * part + sizeof(uint32_t) * part + sizeof(uint32_t) * (kSortWarps * 256 + 512);
@@ -376,13 +376,12 @@ int radix_sort(RmeshCtx* c, K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals
   uint32_t* vout = vals_alt;
   for (int p = 0; p < passes; ++p) {
     onesweep_kernel<K><<<grid, kSortThreads, smem, c->stream>>>(kin, vin, kout, vout, n_ptr, n_is_u64, cap, 8 * p, p,
-                                                                st, c->sort_status.as<unsigned long long>(),
+                                                                st, hist, c->sort_status.as<unsigned long long>(),
                                                                 &cnt->err);
     CKL();
     std::swap(kin, kout);
     std::swap(vin, vout);
   }
-  (void)capturing;
   *out_keys = kin;
   *out_vals = vin;
   return RMESH_OK;
@@ -406,6 +405,29 @@ int setup_sort_attrs() {
 }
 
 // ---------------------------------------------------------------- buffers
+// What a run needs cleared, laid out in one buffer: one memset per run.
+struct RunState {
+  size_t ranges, scan_a, scan_b, hist_a, hist_b, order_hist, tickets, bytes;
+  RunState(uint64_t items, uint32_t total_tiles) {
+    size_t at = 0;
+    auto take = [&](size_t n) {
+      const size_t here = at;
+      at += (n + 255) / 256 * 256;
+      return here;
+    };
+    // chained scans over blocks of kCompactItems items, each with its ticket
+    const size_t scan = ((items + kCompactItems - 1) / kCompactItems + 2) * 8;
+    ranges = take((size_t)std::max<uint32_t>(total_tiles, 1) * 8);
+    scan_a = take(scan);
+    scan_b = take(scan);
+    hist_a = take(sizeof(SortHist));
+    hist_b = take(sizeof(SortHist));
+    order_hist = take(2 * kOrderBuckets * 4 * kMaxTileGroups);
+    tickets = take(kMaxTileGroups * 4);
+    bytes = at;
+  }
+};
+
 int ensure_run_buffers(RmeshCtx* c, int n_views, uint64_t total_pixels, uint32_t total_tiles) {
   const uint64_t items = (uint64_t)n_views * (uint64_t)c->M;
   CKR(ensure_buf(c, c->vis_key, items * 8));
@@ -428,11 +450,8 @@ int ensure_run_buffers(RmeshCtx* c, int n_views, uint64_t total_pixels, uint32_t
   CKR(ensure_buf(c, c->spans_adj, c->cap_pairs * 4 * kSpanWords));
   const uint64_t sort_items = std::max<uint64_t>(std::max<uint64_t>(items, c->cap_pairs), 4ull * c->M);
   CKR(ensure_buf(c, c->sort_status, ((sort_items + kSortPart - 1) / kSortPart + 1) * 256 * 8));
-  CKR(ensure_buf(c, c->scan_status, ((items + 255) / 256 + 2) * 8));
-  CKR(ensure_buf(c, c->ranges, (uint64_t)std::max<uint32_t>(total_tiles, 1) * 8));
+  CKR(ensure_buf(c, c->run_state, RunState(items, total_tiles).bytes));
   CKR(ensure_buf(c, c->tile_order, (uint64_t)std::max<uint32_t>(total_tiles, 1) * 4));
-  CKR(ensure_buf(c, c->order_hist, 2 * kOrderBuckets * 4 * kMaxTileGroups));
-  CKR(ensure_buf(c, c->tickets, kMaxTileGroups * 4));
   CKR(ensure_buf(c, c->rgba, std::max<uint64_t>(total_pixels, 1) * 16));
   return RMESH_OK;
 }
@@ -526,11 +545,14 @@ int run_records(RmeshCtx* c, bool capturing) {
 int run_bin(RmeshCtx* c, const ViewParams* views_dev, int n_views, uint32_t total_tiles, Counters* cnt,
             bool capturing, const std::vector<TileGroup>& groups, bool adjoint = true) {
   const uint64_t items = (uint64_t)n_views * (uint64_t)c->M;
-  // chained scans over blocks of kCompactItems items (key compaction) and
-  // sorted entries (pair offsets)
   const unsigned nscan = (unsigned)((items + kCompactItems - 1) / kCompactItems);
-  unsigned long long* status = c->scan_status.as<unsigned long long>();
-  uint32_t* ticket = reinterpret_cast<uint32_t*>(status + nscan + 1);
+  const RunState rs(items, total_tiles);
+  char* state = c->run_state.as<char>();
+  unsigned long long* scan_a = reinterpret_cast<unsigned long long*>(state + rs.scan_a);
+  unsigned long long* scan_b = reinterpret_cast<unsigned long long*>(state + rs.scan_b);
+  c->ranges = reinterpret_cast<uint2*>(state + rs.ranges);
+  c->tickets = reinterpret_cast<uint32_t*>(state + rs.tickets);
+  CK(cudaMemsetAsync(state, 0, rs.bytes, c->stream));
   {
     StageScope sc(c, kStProject, capturing);
     ProjectArgs pa;
@@ -548,7 +570,6 @@ int run_bin(RmeshCtx* c, const ViewParams* views_dev, int n_views, uint32_t tota
     pa.vis_color = c->vis_color.as<float4>();
     project_kernel<<<(unsigned)((items + 255) / 256), 256, 0, c->stream>>>(pa);
     CKL();
-    CK(cudaMemsetAsync(status, 0, (size_t)(nscan + 2) * 8, c->stream));
     CompactArgs ca;
     ca.M = (int)c->M;
     ca.n_views = n_views;
@@ -557,8 +578,8 @@ int run_bin(RmeshCtx* c, const ViewParams* views_dev, int n_views, uint32_t tota
     ca.vis_cnt = c->vis_cnt.as<uint32_t>();
     ca.vis_key = c->vis_key.as<unsigned long long>();
     ca.vis_val = c->vis_val.as<uint32_t>();
-    ca.status = status;
-    ca.ticket = ticket;
+    ca.status = scan_a;
+    ca.ticket = reinterpret_cast<uint32_t*>(scan_a + nscan + 1);
     ca.counters = cnt;
     compact_keys_kernel<<<nscan, 256, 0, c->stream>>>(ca);
     CKL();
@@ -573,19 +594,19 @@ int run_bin(RmeshCtx* c, const ViewParams* views_dev, int n_views, uint32_t tota
     // gives; the view and tile count ride in the key's high bits
     CKR(radix_sort<unsigned long long>(c, c->vis_key.as<unsigned long long>(), c->vis_val.as<uint32_t>(),
                                        c->vis_key_alt.as<unsigned long long>(), c->vis_val_alt.as<uint32_t>(),
-                                       &cnt->n_vis, 0, items, 32, &tk, &tv, capturing));
+                                       &cnt->n_vis, 0, items, 32, &tk, &tv,
+                                       reinterpret_cast<SortHist*>(state + rs.hist_a)));
   }
   {
     StageScope sc(c, kStEmit, capturing);
-    CK(cudaMemsetAsync(status, 0, (size_t)(nscan + 2) * 8, c->stream));
     EmitScanArgs es;
     es.tet_key_sorted = tk;
     es.tet_val_sorted = tv;
     es.vis_cnt = c->vis_cnt.as<uint32_t>();
     es.n_vis_ptr = &cnt->n_vis;
     es.group_off = c->group_off.as<unsigned long long>();
-    es.status = status;
-    es.ticket = ticket;
+    es.status = scan_b;
+    es.ticket = reinterpret_cast<uint32_t*>(scan_b + nscan + 1);
     es.counters = cnt;
     emit_scan_kernel<<<nscan, 256, 0, c->stream>>>(es);
     CKL();
@@ -609,11 +630,11 @@ int run_bin(RmeshCtx* c, const ViewParams* views_dev, int n_views, uint32_t tota
     const int bits = std::max(1, bitlen(total_tiles));
     CKR(radix_sort<uint32_t>(c, c->pair_key.as<uint32_t>(), c->pair_val.as<uint32_t>(), c->pair_key_alt.as<uint32_t>(),
                              c->pair_val_alt.as<uint32_t>(), &cnt->n_pairs, 1, c->cap_pairs, bits,
-                             &c->sorted_pair_key, &c->sorted_pair_val, capturing));
+                             &c->sorted_pair_key, &c->sorted_pair_val,
+                             reinterpret_cast<SortHist*>(state + rs.hist_b)));
   }
   {
     StageScope sc(c, kStRanges, capturing);
-    CK(cudaMemsetAsync(c->ranges.p, 0, (size_t)total_tiles * 8, c->stream));
     PairSpanArgs sa;
     sa.views = views_dev;
     sa.n_views = n_views;
@@ -625,24 +646,22 @@ int run_bin(RmeshCtx* c, const ViewParams* views_dev, int n_views, uint32_t tota
     sa.spans_fwd = c->spans_fwd.as<uint32_t>();
     sa.spans_adj = adjoint ? c->spans_adj.as<uint32_t>() : nullptr;
     sa.stride = c->cap_pairs;
-    sa.ranges = c->ranges.as<uint2>();
+    sa.ranges = c->ranges;
     sa.counters = cnt;
     const int sblocks = (int)std::min<uint64_t>((c->cap_pairs + 255) / 256, (uint64_t)c->num_sms * 8);
     pair_spans_kernel<<<std::max(1, sblocks), 256, 0, c->stream>>>(sa);
     CKL();
     // longest-first order of each launch's tiles for the persistent tile
     // kernel (indices relative to the launch's first tile)
-    CK(cudaMemsetAsync(c->order_hist.p, 0, 2 * kOrderBuckets * 4 * groups.size(), c->stream));
-    CK(cudaMemsetAsync(c->tickets.p, 0, kMaxTileGroups * 4, c->stream));
     for (size_t gi = 0; gi < groups.size(); ++gi) {
       const TileGroup& g = groups[gi];
       if (g.n_tiles == 0) continue;
-      uint32_t* hist = c->order_hist.as<uint32_t>() + 2 * kOrderBuckets * gi;
+      uint32_t* hist = reinterpret_cast<uint32_t*>(state + rs.order_hist) + 2 * kOrderBuckets * gi;
       const int oblocks =
           (int)std::max<uint64_t>(1, std::min<uint64_t>((g.n_tiles + 255) / 256, (uint64_t)c->num_sms * 2));
-      tile_order_hist_kernel<<<oblocks, 256, 0, c->stream>>>(c->ranges.as<uint2>() + g.tile_lo, g.n_tiles, hist);
+      tile_order_hist_kernel<<<oblocks, 256, 0, c->stream>>>(c->ranges + g.tile_lo, g.n_tiles, hist);
       CKL();
-      tile_order_stable_kernel<<<1, kOrderThreads, 0, c->stream>>>(c->ranges.as<uint2>() + g.tile_lo, g.n_tiles,
+      tile_order_stable_kernel<<<1, kOrderThreads, 0, c->stream>>>(c->ranges + g.tile_lo, g.n_tiles,
                                                                   hist, c->tile_order.as<uint32_t>() + g.tile_lo);
       CKL();
     }
@@ -729,7 +748,7 @@ int launch_groups(RmeshCtx* c, const TileArgs& base, const std::vector<TileGroup
     TileArgs ta = base;
     ta.n_tiles = g.n_tiles;
     ta.tile_lo = g.tile_lo;
-    ta.ticket = c->tickets.as<uint32_t>() + gi;
+    ta.ticket = c->tickets + gi;
     ta.tile_order = c->tile_order.as<uint32_t>() + g.tile_lo;
     CKR((launch_tile_m<MODE, AUX>(c, ta, g.n_tiles, true, g.conf)));
   }
@@ -742,7 +761,7 @@ TileArgs base_tile_args(RmeshCtx* c, const ViewParams* views_dev, int n_views, u
   ta.views = views_dev;
   ta.n_views = n_views;
   ta.n_tiles = n_tiles;
-  ta.ranges = c->ranges.as<uint2>();
+  ta.ranges = c->ranges;
   ta.pair_val = c->sorted_pair_val;
   ta.vis_view = c->vis_view.as<TetView>();
   ta.rec = c->rec.as<TetRec>();
@@ -756,7 +775,7 @@ TileArgs base_tile_args(RmeshCtx* c, const ViewParams* views_dev, int n_views, u
   ta.span_stride = c->cap_pairs;
   ta.tile_order = c->tile_order.as<uint32_t>();
   ta.tile_lo = 0;
-  ta.ticket = c->tickets.as<uint32_t>();
+  ta.ticket = c->tickets;
   return ta;
 }
 
@@ -900,6 +919,7 @@ int train_views(RmeshCtx* c, const RmeshCamera* cams, int n_views, const float* 
   const int run_views = plain ? 1 : n_views;
   const bool direct_gt = is_device_ptr(gt);
   for (int attempt = 0; attempt < 4; ++attempt) {
+    c->have_forward = false;  // the run's buffers may move
     CKR(ensure_run_buffers(c, run_views, total_pix, plain ? max_tiles : total_tiles));
     CKR(ensure_moments(c, run_views));
     if (!direct_gt) CKR(ensure_buf(c, c->gt, total_pix * 12));
@@ -1030,11 +1050,13 @@ int build_csr(RmeshCtx* c) {
   const uint64_t n_refs = 4ull * (uint64_t)c->M;
   CKR(ensure_buf(c, c->csr_off, (c->N + 1) * 4));
   CKR(ensure_buf(c, c->csr_ref, n_refs * 4));
-  DevBuf k0, k1, v1, nbuf;
+  DevBuf k0, k1, v1, nbuf, hist;
   CKR(ensure_buf(c, k0, n_refs * 4));
   CKR(ensure_buf(c, k1, n_refs * 4));
   CKR(ensure_buf(c, v1, n_refs * 4));
   CKR(ensure_buf(c, nbuf, 8));
+  CKR(ensure_buf(c, hist, sizeof(SortHist)));
+  CK(cudaMemsetAsync(hist.p, 0, sizeof(SortHist), c->stream));
   const uint32_t n32 = (uint32_t)n_refs;
   CK(cudaMemcpyAsync(nbuf.p, &n32, 4, cudaMemcpyHostToDevice, c->stream));
   csr_fill_kernel<<<(unsigned)((n_refs + 255) / 256), 256, 0, c->stream>>>((int)c->M, c->idx.as<uint32_t>(),
@@ -1046,7 +1068,7 @@ int build_csr(RmeshCtx* c) {
   uint32_t* ok_vals = nullptr;
   CKR(radix_sort<uint32_t>(c, k0.as<uint32_t>(), c->csr_ref.as<uint32_t>(), k1.as<uint32_t>(), v1.as<uint32_t>(),
                            nbuf.p, 0, n_refs, std::max(1, bitlen((uint64_t)std::max<int64_t>(c->N - 1, 1))), &ok_keys,
-                           &ok_vals, false));
+                           &ok_vals, hist.as<SortHist>()));
   if (ok_vals != c->csr_ref.as<uint32_t>())
     CK(cudaMemcpyAsync(c->csr_ref.p, ok_vals, n_refs * 4, cudaMemcpyDeviceToDevice, c->stream));
   csr_offsets_kernel<<<(unsigned)((n_refs + 1 + 255) / 256), 256, 0, c->stream>>>((int)n_refs, (int)c->N, ok_keys,
@@ -1364,12 +1386,12 @@ int rmesh_get_info(RmeshCtx* c, RmeshInfo* info) {
   DevBuf* all[] = {&c->verts, &c->idx, &c->dens, &c->cgrad, &c->base, &c->circ, &c->m_verts, &c->v_verts,
                    &c->m_dens, &c->v_dens, &c->m_cgrad, &c->v_cgrad, &c->m_base, &c->v_base, &c->rec,
                    &c->color4, &c->grad_slot, &c->csr_off, &c->csr_ref, &c->views_d, &c->counters_d, &c->hp_d,
-                   &c->sort_state, &c->sort_status, &c->scan_status, &c->vis_key, &c->vis_val, &c->group_off,
+                   &c->sort_state, &c->sort_status, &c->run_state, &c->vis_key, &c->vis_val, &c->group_off,
                    &c->vis_cnt, &c->vis_proj, &c->vis_view, &c->vis_key_alt, &c->vis_val_alt, &c->pair_key,
-                   &c->pair_val, &c->pair_key_alt, &c->pair_val_alt, &c->ranges, &c->rgba, &c->aux, &c->dl,
+                   &c->pair_val, &c->pair_key_alt, &c->pair_val_alt, &c->rgba, &c->aux, &c->dl,
                    &c->gt, &c->out_a, &c->out_b, &c->out_c, &c->out_d, &c->sh, &c->m_sh, &c->v_sh,
                    &c->vis_color, &c->mom, &c->err_in, &c->err_out, &c->aux_data, &c->dl_aux, &c->d_aux,
-                   &c->spans_fwd, &c->spans_adj, &c->tile_order, &c->order_hist, &c->tickets};
+                   &c->spans_fwd, &c->spans_adj, &c->tile_order};
   for (DevBuf* b : all) info->device_bytes += b->bytes;
   return RMESH_OK;
 }
@@ -1433,6 +1455,7 @@ int rmesh_forward_views(RmeshCtx* c, const RmeshCamera* cams, int32_t n_views, f
   const uint32_t total_tiles = pl.total_tiles;
   const uint64_t aux_floats = total_pix * (8 + (uint64_t)c->aux_dim);
   for (int attempt = 0; attempt < 4; ++attempt) {
+    c->have_forward = false;  // the run's buffers may move
     CKR(ensure_run_buffers(c, n_views, total_pix, total_tiles));
     if (aux_out) CKR(ensure_buf(c, c->aux, aux_floats * 4));
     CKR(upload_views(c, n_views));
@@ -1476,6 +1499,7 @@ int rmesh_forward_tiled(RmeshCtx* c, const RmeshCamera* cam, float* rgba_out, fl
     CKR(fill_view(c, *cam, c->views_h[0], 0, 0, tc));
     const uint32_t tiles = (uint32_t)(c->views_h[0].tiles_x * c->views_h[0].tiles_y);
     const std::vector<TileGroup> one{TileGroup{tc, 0u, tiles}};
+    c->have_forward = false;  // the run's buffers may move
     CKR(ensure_run_buffers(c, 1, npix, tiles));
     if (aux_out) CKR(ensure_buf(c, c->aux, npix * (8 + (uint64_t)c->aux_dim) * 4));
     CKR(upload_views(c, 1));
@@ -1533,7 +1557,7 @@ static int backward_impl(RmeshCtx* c, const float* dl, const float* dl_aux, floa
     CK(cudaMemsetAsync(c->d_aux.p, 0, (uint64_t)c->M * c->aux_dim * 4, c->stream));
   }
   Counters* cnt = c->counters_d.as<Counters>();
-  CK(cudaMemsetAsync(c->tickets.p, 0, kMaxTileGroups * 4, c->stream));
+  CK(cudaMemsetAsync(c->tickets, 0, kMaxTileGroups * 4, c->stream));
   const std::vector<TileGroup> one{TileGroup{TileConf{c->last_ts, c->last_wide}, 0u, c->last_tiles}};
   ViewParams* vd = c->views_d.as<ViewParams>();
   CKR(ensure_moments(c, 1));
@@ -1604,7 +1628,7 @@ int rmesh_forward_error(RmeshCtx* c, const float* pixel_err, const float* ssim_e
   CKR(ensure_moments(c, 1));
   CK(cudaMemsetAsync(c->mom.p, 0, M * kErrMom * 4, c->stream));
   Counters* cnt = c->counters_d.as<Counters>();
-  CK(cudaMemsetAsync(c->tickets.p, 0, kMaxTileGroups * 4, c->stream));
+  CK(cudaMemsetAsync(c->tickets, 0, kMaxTileGroups * 4, c->stream));
   const std::vector<TileGroup> one{TileGroup{TileConf{c->last_ts, c->last_wide}, 0u, c->last_tiles}};
   ViewParams* vd = c->views_d.as<ViewParams>();
   {
@@ -1846,7 +1870,7 @@ int rmesh_debug_ranges(RmeshCtx* c, uint32_t* ranges, uint64_t n_tiles) {
   DevGuard dg__(c);
   if (!c->have_forward) return fail(c, RMESH_ERR_STATE, "no forward yet");
   const uint64_t k = std::min<uint64_t>(n_tiles, c->last_tiles);
-  CK(cudaMemcpyAsync(ranges, c->ranges.p, k * 8, cudaMemcpyDefault, c->stream));
+  CK(cudaMemcpyAsync(ranges, c->ranges, k * 8, cudaMemcpyDefault, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   return RMESH_OK;
 }

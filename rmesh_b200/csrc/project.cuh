@@ -156,7 +156,7 @@ __device__ __forceinline__ void scanline_tiles(const float px[4], const float py
 //           the opposite vertex, and num = dot(n, va - cam), explicitly rounded
 //           (rasterize_compute.wgsl:301-314, 360-372)
 //   cb      colour + dot(g, cam - v0) (the base colour at the camera, :395-396), density
-//   gm      colour gradient g; w = face flip bits (bit f) | behind (bit 4) |
+//   gm      colour gradient g; w = face flip bits (bit f) |
 //           kPlainPlanes: every |n| component is at most 2^58 and every num is 0
 //           or 2^-60 <= |num| <= 2^60, so that with |den| >= 1e-20 the tile
 //           kernel's fused division keeps all its intermediates in range
@@ -199,17 +199,14 @@ __device__ __forceinline__ void write_tet_view(TetView* dst, const TetRec& r, co
   const float boff = dot3x(gx, gy, gz, fs(camx, r.a.x), fs(camy, r.a.y), fs(camz, r.a.z));
   out.cb = make_float4(fa(col.x, boff), fa(col.y, boff), fa(col.z, boff), r.a.w);
   float qx[4], qy[4];
-  bool behind = false;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     float c[4];
     clip_exact(V.vp, vs[k].x, vs[k].y, vs[k].z, c);
-    behind = behind || (c[3] <= 0.0f);
     const float iw = __fdividef(1.0f, c[3]);
     qx[k] = (c[0] * iw + 1.0f) * 0.5f * V.Wf;
     qy[k] = (1.0f - c[1] * iw) * 0.5f * V.Hf;
   }
-  if (behind) flags |= 1u << 4;
   out.gm = make_float4(gx, gy, gz, __uint_as_float(flags));
   out.px = make_float4(qx[0], qx[1], qx[2], qx[3]);
   out.py = make_float4(qy[0], qy[1], qy[2], qy[3]);

@@ -3,7 +3,7 @@
 // Replaces the reference's 3-kernel-per-pass DeviceRadixSort
 // (crates/rmesh-sort/src/drs.rs:180-279, wgsl/drs_{upsweep,scan,downsweep}.wgsl):
 // one histogram kernel computes the digit counts of every pass in a single
-// read of the keys, then each pass is ONE kernel that ranks a 4096-key
+// read of the keys (each partition scans its pass's 256 counts itself), then each pass is ONE kernel that ranks a 4096-key
 // partition in shared memory (warp multi-split: peers of a digit found by one
 // ballot per digit bit), looks back
 // across earlier partitions for the per-digit global offset, and scatters
@@ -34,10 +34,12 @@ struct SortCfg {
 constexpr int kMaxPasses = 8;
 
 struct SortState {
-  uint32_t epoch;                       // bumped once per sort
-  uint32_t ticket[kMaxPasses];          // partition tickets, reset by sort_scan_kernel
-  uint32_t hist[kMaxPasses][256];       // global digit counts (zeroed by a memset per sort)
-  uint32_t offs[kMaxPasses][256];       // exclusive digit offsets
+  uint32_t epoch;                // bumped once per sort (sort_hist_kernel)
+  uint32_t ticket[kMaxPasses];   // partition tickets, reset by sort_hist_kernel
+};
+// Global digit counts of a sort's passes (zeroed before the sort).
+struct SortHist {
+  uint32_t count[kMaxPasses][256];
 };
 
 template <typename K>
@@ -45,12 +47,17 @@ __device__ __forceinline__ uint32_t digit_of(K key, int shift) {
   return (uint32_t)(key >> shift) & 0xFFu;
 }
 
-// One read of the keys; counts digits of all passes.
+// One read of the keys; counts digits of all passes.  Its first block also bumps
+// the epoch and resets the tickets for the passes that follow.
 template <typename K>
 __global__ void __launch_bounds__(256) sort_hist_kernel(const K* __restrict__ keys, const void* n_ptr, int n_is_u64,
                                                         unsigned long long cap, int begin_bit, int passes,
-                                                        SortState* st) {
+                                                        SortState* st, SortHist* hist) {
   __shared__ uint32_t h[kMaxPasses][256];
+  if (blockIdx.x == 0) {
+    if (threadIdx.x < kMaxPasses) st->ticket[threadIdx.x] = 0u;
+    if (threadIdx.x == 0) st->epoch = st->epoch + 1u;
+  }
   for (int i = threadIdx.x; i < kMaxPasses * 256; i += blockDim.x) (&h[0][0])[i] = 0u;
   __syncthreads();
   unsigned long long n = n_is_u64 ? *(const unsigned long long*)n_ptr : *(const uint32_t*)n_ptr;
@@ -63,29 +70,37 @@ __global__ void __launch_bounds__(256) sort_hist_kernel(const K* __restrict__ ke
   __syncthreads();
   for (int i = threadIdx.x; i < passes * 256; i += blockDim.x) {
     const uint32_t c = (&h[0][0])[i];
-    if (c) atomicAdd(&st->hist[0][0] + i, c);
+    if (c) atomicAdd(&hist->count[0][0] + i, c);
   }
 }
 
-// Exclusive scan of each pass's 256 digit counts; bumps the epoch; resets tickets.
-__global__ void sort_scan_kernel(int passes, SortState* st) {
-  __shared__ uint32_t s[256];
-  const int d = threadIdx.x;  // 256 threads
-  for (int p = 0; p < passes; ++p) {
-    s[d] = st->hist[p][d];
-    __syncthreads();
-    // Hillis-Steele inclusive scan
-    for (int o = 1; o < 256; o <<= 1) {
-      const uint32_t v = d >= o ? s[d - o] : 0u;
-      __syncthreads();
-      s[d] += v;
-      __syncthreads();
+// Exclusive scans over the block's 256 threads of two values at once (one
+// shuffle scan per warp, one barrier pair); `warps`: 2 x kSortWarps words.
+__device__ __forceinline__ void block_scan2(uint32_t a, uint32_t b, uint32_t* warps, uint32_t& ea, uint32_t& eb) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t x = a, y = b;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t u = __shfl_up_sync(0xffffffffu, x, o), v = __shfl_up_sync(0xffffffffu, y, o);
+    if (lane >= o) {
+      x += u;
+      y += v;
     }
-    st->offs[p][d] = s[d] - st->hist[p][d];
-    __syncthreads();
   }
-  if (d < kMaxPasses) st->ticket[d] = 0u;
-  if (d == 0) st->epoch = st->epoch + 1u;
+  if (lane == 31) {
+    warps[warp] = x;
+    warps[kSortWarps + warp] = y;
+  }
+  __syncthreads();
+  ea = x - a;
+  eb = y - b;
+#pragma unroll
+  for (int w = 0; w < kSortWarps; ++w) {
+    if (w < warp) {
+      ea += warps[w];
+      eb += warps[kSortWarps + w];
+    }
+  }
 }
 
 // Status word: [63:32] epoch, [31:30] flag (1 aggregate, 2 inclusive), [29:0] count.
@@ -99,8 +114,8 @@ __global__ void __launch_bounds__(kSortThreads) onesweep_kernel(const K* __restr
                                                                 K* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
                                                                 const void* n_ptr, int n_is_u64,
                                                                 unsigned long long cap, int shift, int pass,
-                                                                SortState* st, unsigned long long* status,
-                                                                uint32_t* err) {
+                                                                SortState* st, const SortHist* hist,
+                                                                unsigned long long* status, uint32_t* err) {
   extern __shared__ __align__(16) unsigned char smem[];
   K* s_keys = reinterpret_cast<K*>(smem);
   uint32_t* s_vals = reinterpret_cast<uint32_t*>(smem + sizeof(K) * SortCfg<K>::PART);
@@ -199,20 +214,12 @@ __global__ void __launch_bounds__(kSortThreads) onesweep_kernel(const K* __restr
     __threadfence();
     st_volatile_u64(my, pack_status(epoch, 2u, prefix + cnt));
   }
-  s_gbase[d] = st->offs[pass][d] + prefix;
-
-  // block exclusive scan of cnt over digits -> start of each digit inside the partition
-  s_dstart[d] = cnt;
-  __syncthreads();
-  for (int o = 1; o < 256; o <<= 1) {
-    const uint32_t t = d >= (uint32_t)o ? s_dstart[d - o] : 0u;
-    __syncthreads();
-    s_dstart[d] += t;
-    __syncthreads();
-  }
-  const uint32_t incl = s_dstart[d];
-  __syncthreads();
-  s_dstart[d] = incl - cnt;
+  // digit d's start over all keys and inside the partition
+  __shared__ uint32_t s_warp[2 * kSortWarps];
+  uint32_t global_start, part_start;
+  block_scan2(hist->count[pass][d], cnt, s_warp, global_start, part_start);
+  s_gbase[d] = global_start + prefix;
+  s_dstart[d] = part_start;
   __syncthreads();
 
   // scatter into shared memory in sorted order

@@ -1200,8 +1200,8 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : (TS == 16 || MODE 
 
 // Span words of every sorted (tile, tet) pair, one set per rule: a byte per tile
 // row (pack_span, row_spans), four rows per 32-bit word, over the rows its tet
-// reaches; a strip of the tile kernel reads the word of its rows.  Other rows,
-// tets with a vertex behind the camera and sentinel slots get empty spans.  Each
+// reaches; a strip of the tile kernel reads the word of its rows.  Other rows and
+// sentinel slots get empty spans.  Each
 // warp takes 32 consecutive pairs; lane l sets up pair l (sorted vertices, edge
 // slopes) in shared memory, and the warp's (pair, row) tasks are spread over its
 // lanes through a prefix of the row counts, so lanes stay busy whatever the rows
@@ -1265,7 +1265,7 @@ __global__ void __launch_bounds__(256) pair_spans_kernel(PairSpanArgs a) {
       st.valid_cols = min(TS, V.W - (int)(tx * (uint32_t)TS));
       const int valid_rows = min(TS, V.H - (int)(ty * (uint32_t)TS));
       const TetView* tv = a.vis_view + a.vals[p];
-      if (!((__float_as_uint(__ldg(&tv->gm.w)) >> 4) & 1u)) {
+      {  // (a tet with a vertex behind the camera has no pairs)
         const float4 gx4 = __ldg(&tv->px), gy4 = __ldg(&tv->py);
         const float tile_ox = (float)(tx * (uint32_t)TS), tile_oy = (float)(ty * (uint32_t)TS);
         st.x[0] = gx4.x - tile_ox; st.x[1] = gx4.y - tile_ox; st.x[2] = gx4.z - tile_ox; st.x[3] = gx4.w - tile_ox;
