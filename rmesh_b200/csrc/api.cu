@@ -622,7 +622,8 @@ int run_bin(RmeshCtx* c, const ViewParams* views_dev, int n_views, uint32_t tota
     ea.pair_val = c->pair_val.as<uint32_t>();
     ea.cap = c->cap_pairs;
     ea.counters = cnt;
-    emit_kernel<<<(unsigned)((items + 255) / 256), 256, 0, c->stream>>>(ea);
+    // at least eight blocks per SM, for views with few entries (emit_kernel's split)
+    emit_kernel<<<(unsigned)std::max<uint64_t>((items + 255) / 256, (uint64_t)c->num_sms * 8), 256, 0, c->stream>>>(ea);
     CKL();
   }
   {

@@ -41,9 +41,10 @@ __global__ void __launch_bounds__(256) build_records_kernel(int M, const float* 
 
 // Conservative scanline over tile rows (project_compute.wgsl:202-259 ==
 // tile_gen_scan_compute.wgsl:119-201), exact arithmetic.  tile_range gives a
-// tet's clamped pixel box in tiles (false when it is empty), tile_row_span one
-// tile row's [tx0, tx1] (false when the row is empty); scanline_tiles calls
-// f(ty, tx0, tx1) for every tile row with a non-empty clamped span.
+// tet's clamped pixel box in tiles (false when it is empty), boundary_cross the
+// crossings of one row boundary, row_span one tile row's [tx0, tx1] from its two
+// boundaries' (false when the row is empty); scanline_tiles calls f(ty, tx0, tx1)
+// for every tile row with a non-empty clamped span.
 struct TileBox {
   uint32_t min_x, max_x, min_y, max_y;
 };
@@ -60,41 +61,6 @@ __device__ __forceinline__ bool tile_range(const float px[4], const float py[4],
   tb.max_x = min(__float2uint_rz(fdv(pix_max_x, T)), tiles_x_total - 1u);
   tb.min_y = __float2uint_rz(fdv(pix_min_y, T));
   tb.max_y = min(__float2uint_rz(fdv(pix_max_y, T)), __float2uint_rz(ceilf(fdv(H, T))) - 1u);
-  return true;
-}
-__device__ __forceinline__ bool tile_row_span(const float px[4], const float py[4], uint32_t TS, const TileBox& tb,
-                                              uint32_t ty, uint32_t& tx0, uint32_t& tx1) {
-  const float T = (float)TS;
-  const int ei[6] = {0, 0, 0, 1, 1, 2};
-  const int ej[6] = {1, 2, 3, 2, 3, 3};
-  float xl = 1e10f, xr = -1e10f;
-#pragma unroll
-  for (int e = 0; e < 6; ++e) {
-    const float yi = py[ei[e]], yj = py[ej[e]], xi = px[ei[e]], xj = px[ej[e]];
-#pragma unroll
-    for (uint32_t b = 0; b < 2; ++b) {
-      const float ytest = fm((float)(ty + b), T);
-      if ((yi <= ytest && yj > ytest) || (yj <= ytest && yi > ytest)) {
-        const float t = fdv(fs(ytest, yi), fs(yj, yi));
-        const float x = fa(xi, fm(t, fs(xj, xi)));
-        xl = fminf(xl, x);
-        xr = fmaxf(xr, x);
-      }
-    }
-  }
-  const float band_lo = fm((float)ty, T), band_hi = fm((float)(ty + 1u), T);
-#pragma unroll
-  for (int v = 0; v < 4; ++v) {
-    if (py[v] >= band_lo && py[v] <= band_hi) {
-      xl = fminf(xl, px[v]);
-      xr = fmaxf(xr, px[v]);
-    }
-  }
-  if (!(xl <= xr)) return false;
-  tx0 = __float2uint_rz(fmaxf(floorf(fdv(xl, T)), 0.0f));
-  tx1 = __float2uint_rz(fmaxf(floorf(fdv(xr, T)), 0.0f));
-  tx0 = min(max(tx0, tb.min_x), tb.max_x);
-  tx1 = min(max(tx1, tb.min_x), tb.max_x);
   return true;
 }
 // Crossings of the tet's edges with the row boundary y = row * TS.
@@ -114,9 +80,29 @@ __device__ __forceinline__ void boundary_cross(const float px[4], const float py
     }
   }
 }
-// f(ty, tx0, tx1) for every tile row with a non-empty clamped span: tile_row_span
-// of each row, walked downwards so that a boundary's crossings (a third of them
-// exact divisions) are taken once for the two rows that share it.
+// Tile columns of row ty: xl / xr are the crossings of its two boundaries, to which
+// the vertices inside the row's band are added.
+__device__ __forceinline__ bool row_span(const float px[4], const float py[4], float xl, float xr, uint32_t TS,
+                                         const TileBox& tb, uint32_t ty, uint32_t& tx0, uint32_t& tx1) {
+  const float T = (float)TS;
+  const float band_lo = fm((float)ty, T), band_hi = fm((float)(ty + 1u), T);
+#pragma unroll
+  for (int v = 0; v < 4; ++v) {
+    if (py[v] >= band_lo && py[v] <= band_hi) {
+      xl = fminf(xl, px[v]);
+      xr = fmaxf(xr, px[v]);
+    }
+  }
+  if (!(xl <= xr)) return false;
+  tx0 = __float2uint_rz(fmaxf(floorf(fdv(xl, T)), 0.0f));
+  tx1 = __float2uint_rz(fmaxf(floorf(fdv(xr, T)), 0.0f));
+  tx0 = min(max(tx0, tb.min_x), tb.max_x);
+  tx1 = min(max(tx1, tb.min_x), tb.max_x);
+  return true;
+}
+// f(ty, tx0, tx1) for every tile row with a non-empty clamped span, walked
+// downwards so that a boundary's crossings (exact divisions) are taken once for
+// the two rows that share it.
 template <class F>
 __device__ __forceinline__ void scanline_tiles(const float px[4], const float py[4], float W, float H, uint32_t TS,
                                                F&& f) {
@@ -126,25 +112,12 @@ __device__ __forceinline__ void scanline_tiles(const float px[4], const float py
   float al, ar;
   boundary_cross(px, py, fm((float)tb.min_y, T), al, ar);
   for (uint32_t ty = tb.min_y; ty <= tb.max_y; ++ty) {
-    const float band_lo = fm((float)ty, T), band_hi = fm((float)(ty + 1u), T);
     float bl, br;
-    boundary_cross(px, py, band_hi, bl, br);
-    float xl = fminf(al, bl), xr = fmaxf(ar, br);
+    boundary_cross(px, py, fm((float)(ty + 1u), T), bl, br);
+    uint32_t tx0, tx1;
+    if (row_span(px, py, fminf(al, bl), fmaxf(ar, br), TS, tb, ty, tx0, tx1)) f(ty, tx0, tx1);
     al = bl;
     ar = br;
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      if (py[v] >= band_lo && py[v] <= band_hi) {
-        xl = fminf(xl, px[v]);
-        xr = fmaxf(xr, px[v]);
-      }
-    }
-    if (!(xl <= xr)) continue;
-    uint32_t tx0 = __float2uint_rz(fmaxf(floorf(fdv(xl, T)), 0.0f));
-    uint32_t tx1 = __float2uint_rz(fmaxf(floorf(fdv(xr, T)), 0.0f));
-    tx0 = min(max(tx0, tb.min_x), tb.max_x);
-    tx1 = min(max(tx1, tb.min_x), tb.max_x);
-    f(ty, tx0, tx1);
   }
 }
 
