@@ -87,6 +87,9 @@ struct RmeshCtx {
   int device = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
+  // host targets of a step are copied on their own stream beside the binning
+  cudaStream_t copy_stream = nullptr;
+  cudaEvent_t copy_begin = nullptr, copy_done = nullptr;
   int64_t N = 0, M = 0;
   int width = 0, height = 0, tile_size = 12;
   int tile_wide = 0;  // default tile configuration: tile_size, threads per tile doubled when set
@@ -830,8 +833,15 @@ int run_sh_backward(RmeshCtx* c, const ViewParams* views_dev, int n_views, bool 
   return RMESH_OK;
 }
 
-int sync_counters(RmeshCtx* c, int n) {
+// Counters of a run: enqueue_counters orders their copy behind the run,
+// sync_counters waits for the stream (with whatever was enqueued since) and
+// evaluates them.
+int enqueue_counters(RmeshCtx* c, int n) {
   CK(cudaMemcpyAsync(c->counters_h, c->counters_d.p, sizeof(Counters) * n, cudaMemcpyDeviceToHost, c->stream));
+  return RMESH_OK;
+}
+int sync_counters(RmeshCtx* c, int n, bool enqueued = false) {
+  if (!enqueued) CKR(enqueue_counters(c, n));
   CK(cudaStreamSynchronize(c->stream));
   uint32_t bits = 0;
   uint64_t nv = 0, np = 0;
@@ -938,7 +948,29 @@ int train_views(RmeshCtx* c, const RmeshCamera* cams, int n_views, const float* 
     CK(cudaMemcpyAsync(c->hp_d.p, c->hp_h, sizeof(AdamParams), cudaMemcpyHostToDevice, c->stream));
     CKR(upload_views(c, n_views));
     const float* gt_dev = direct_gt ? gt : c->gt.as<float>();
-    if (!direct_gt) CK(cudaMemcpyAsync(c->gt.p, gt, total_pix * 12, cudaMemcpyHostToDevice, c->stream));
+    // host targets: a replayed graph needs them before its launch; otherwise they
+    // are copied on a second stream once the binning that does not read them is
+    // enqueued (after work the caller ordered on the context's stream before)
+    const bool beside = !direct_gt && mode != RMESH_MODE_GRAPH;
+    if (!direct_gt && !beside) CK(cudaMemcpyAsync(c->gt.p, gt, total_pix * 12, cudaMemcpyHostToDevice, c->stream));
+    if (beside) {
+      if (!c->copy_stream) {
+        CK(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
+        CK(cudaEventCreateWithFlags(&c->copy_begin, cudaEventDisableTiming));
+        CK(cudaEventCreateWithFlags(&c->copy_done, cudaEventDisableTiming));
+      }
+      CK(cudaEventRecord(c->copy_begin, c->stream));
+      CK(cudaStreamWaitEvent(c->copy_stream, c->copy_begin, 0));
+    }
+    bool copied = false;
+    auto need_targets = [&]() -> int {
+      if (!beside || copied) return RMESH_OK;
+      copied = true;
+      CK(cudaMemcpyAsync(c->gt.p, gt, total_pix * 12, cudaMemcpyHostToDevice, c->copy_stream));
+      CK(cudaEventRecord(c->copy_done, c->copy_stream));
+      CK(cudaStreamWaitEvent(c->stream, c->copy_done, 0));
+      return RMESH_OK;
+    };
 
     const int n_cnt = plain ? n_views : 1;
     auto enqueue = [&](bool capturing) -> int {
@@ -954,6 +986,7 @@ int train_views(RmeshCtx* c, const RmeshCamera* cams, int n_views, const float* 
           const std::vector<TileGroup> one{TileGroup{tc, 0u, vt}};
           CKR(run_bin(c, vd + i, 1, vt, cnt + i, capturing, one));
           CKR(clear_moments(c, 1));
+          CKR(need_targets());
           {
             StageScope sc(c, kStComposite, capturing);
             TileArgs ta = base_tile_args(c, vd + i, 1, vt, cnt + i);
@@ -966,6 +999,7 @@ int train_views(RmeshCtx* c, const RmeshCamera* cams, int n_views, const float* 
       } else {
         CKR(run_bin(c, vd, n_views, total_tiles, cnt, capturing, pl.groups));
         CKR(clear_moments(c, n_views));
+        CKR(need_targets());
         {
           StageScope sc(c, kStComposite, capturing);
           TileArgs ta = base_tile_args(c, vd, n_views, total_tiles, cnt);
@@ -1231,6 +1265,9 @@ int rmesh_destroy(RmeshCtx* c) {
     cudaEventDestroy(e.b);
   }
   for (auto e : c->event_pool) cudaEventDestroy(e);
+  if (c->copy_begin) cudaEventDestroy(c->copy_begin);
+  if (c->copy_done) cudaEventDestroy(c->copy_done);
+  if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
   if (c->views_h) cudaFreeHost(c->views_h);
   if (c->counters_h) cudaFreeHost(c->counters_h);
   if (c->hp_h) cudaFreeHost(c->hp_h);
@@ -1478,12 +1515,13 @@ int rmesh_forward_views(RmeshCtx* c, const RmeshCamera* cams, int32_t n_views, f
         CKR((launch_groups<kModeForward, false>(c, ta, pl.groups)));
       }
     }
-    CKR(sync_counters(c, 1));
-    if ((c->last_err_bits & kErrPairOverflow) && grow_pairs(c)) continue;
-    CKR(status_from_bits(c));
+    // one wait for counters and images (an overflowed run writes them again)
+    CKR(enqueue_counters(c, 1));
     CK(cudaMemcpyAsync(rgba_out, c->rgba.p, total_pix * 16, cudaMemcpyDefault, c->stream));
     if (aux_out) CK(cudaMemcpyAsync(aux_out, c->aux.p, aux_floats * 4, cudaMemcpyDefault, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    CKR(sync_counters(c, 1, true));
+    if ((c->last_err_bits & kErrPairOverflow) && grow_pairs(c)) continue;
+    CKR(status_from_bits(c));
     c->have_forward = false;
     c->last_views = n_views;
     return RMESH_OK;
@@ -1522,12 +1560,13 @@ int rmesh_forward_tiled(RmeshCtx* c, const RmeshCamera* cam, float* rgba_out, fl
         CKR((launch_groups<kModeForward, false>(c, ta, one)));
       }
     }
-    CKR(sync_counters(c, 1));
-    if ((c->last_err_bits & kErrPairOverflow) && grow_pairs(c)) continue;
-    CKR(status_from_bits(c));
+    // one wait for counters and image (an overflowed run writes it again)
+    CKR(enqueue_counters(c, 1));
     CK(cudaMemcpyAsync(rgba_out, c->rgba.p, npix * 16, cudaMemcpyDefault, c->stream));
     if (aux_out) CK(cudaMemcpyAsync(aux_out, c->aux.p, npix * (8 + (uint64_t)c->aux_dim) * 4, cudaMemcpyDefault, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    CKR(sync_counters(c, 1, true));
+    if ((c->last_err_bits & kErrPairOverflow) && grow_pairs(c)) continue;
+    CKR(status_from_bits(c));
     c->have_forward = true;
     c->last_tiles = tiles;
     c->last_views = 1;
