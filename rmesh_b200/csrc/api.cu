@@ -532,21 +532,25 @@ int make_plan(RmeshCtx* c, const RmeshCamera* cams, int n_views, bool plain, Vie
 }
 
 // ---------------------------------------------------------------- stages
+RecordArgs record_args(RmeshCtx* c) {
+  return RecordArgs{c->verts.as<float>(), c->idx.as<uint4>(), c->dens.as<float>(), c->cgrad.as<float>(),
+                    c->base.as<float>(),  c->rec.as<TetRec>(), c->color4.as<float4>()};
+}
+// tet records of the run's parameters (a run of one view gathers them in its
+// projection instead, see run_bin)
 int run_records(RmeshCtx* c, bool capturing) {
   StageScope sc(c, kStRecords, capturing);
   const int M = (int)c->M;
-  build_records_kernel<<<(M + 255) / 256, 256, 0, c->stream>>>(M, c->verts.as<float>(), c->idx.as<uint4>(),
-                                                               c->dens.as<float>(), c->cgrad.as<float>(),
-                                                               c->base.as<float>(), c->rec.as<TetRec>(),
-                                                               c->color4.as<float4>());
+  build_records_kernel<<<(M + 255) / 256, 256, 0, c->stream>>>(M, record_args(c));
   CKL();
   return RMESH_OK;
 }
 
 // project -> tet sort -> emit -> pair sort -> ranges for n_views views at views_dev
-// (adjoint: the run's lists will also be walked by the adjoint)
+// (adjoint: the run's lists will also be walked by the adjoint; build: the
+// projection gathers the tet records, for runs of one view)
 int run_bin(RmeshCtx* c, const ViewParams* views_dev, int n_views, uint32_t total_tiles, Counters* cnt,
-            bool capturing, const std::vector<TileGroup>& groups, bool adjoint = true) {
+            bool capturing, const std::vector<TileGroup>& groups, bool adjoint, bool build) {
   const uint64_t items = (uint64_t)n_views * (uint64_t)c->M;
   const unsigned nscan = (unsigned)((items + kCompactItems - 1) / kCompactItems);
   const RunState rs(items, total_tiles);
@@ -567,7 +571,8 @@ int run_bin(RmeshCtx* c, const ViewParams* views_dev, int n_views, uint32_t tota
     pa.vis_proj = c->vis_proj.as<float4>();
     pa.vis_view = c->vis_view.as<TetView>();
     pa.color4 = c->color4.as<float4>();
-    pa.color_view_stride = 0;
+    pa.build = build ? 1 : 0;
+    pa.records = record_args(c);
     pa.sh = c->sh_degree >= 0 ? c->sh.as<float>() : nullptr;
     pa.sh_degree = c->sh_degree;
     pa.vis_color = c->vis_color.as<float4>();
@@ -661,10 +666,11 @@ int run_bin(RmeshCtx* c, const ViewParams* views_dev, int n_views, uint32_t tota
       const TileGroup& g = groups[gi];
       if (g.n_tiles == 0) continue;
       uint32_t* hist = reinterpret_cast<uint32_t*>(state + rs.order_hist) + 2 * kOrderBuckets * gi;
-      const int oblocks =
-          (int)std::max<uint64_t>(1, std::min<uint64_t>((g.n_tiles + 255) / 256, (uint64_t)c->num_sms * 2));
-      tile_order_hist_kernel<<<oblocks, 256, 0, c->stream>>>(c->ranges + g.tile_lo, g.n_tiles, hist);
-      CKL();
+      if (g.n_tiles > kOrderSelfCount) {
+        const int oblocks = (int)std::min<uint64_t>((g.n_tiles + 255) / 256, (uint64_t)c->num_sms * 2);
+        tile_order_hist_kernel<<<oblocks, 256, 0, c->stream>>>(c->ranges + g.tile_lo, g.n_tiles, hist);
+        CKL();
+      }
       tile_order_stable_kernel<<<1, kOrderThreads, 0, c->stream>>>(c->ranges + g.tile_lo, g.n_tiles,
                                                                   hist, c->tile_order.as<uint32_t>() + g.tile_lo);
       CKL();
@@ -977,14 +983,15 @@ int train_views(RmeshCtx* c, const RmeshCamera* cams, int n_views, const float* 
       Counters* cnt = c->counters_d.as<Counters>();
       CK(cudaMemsetAsync(cnt, 0, sizeof(Counters) * n_cnt, c->stream));
       CK(cudaMemsetAsync(c->grad_slot.p, 0, grad_floats(c) * 4, c->stream));
-      CKR(run_records(c, capturing));
+      const bool build = !plain && n_views == 1;
+      if (!build) CKR(run_records(c, capturing));
       ViewParams* vd = c->views_d.as<ViewParams>();
       if (plain) {
         for (int i = 0; i < n_views; ++i) {
           const uint32_t vt = (uint32_t)(c->views_h[i].tiles_x * c->views_h[i].tiles_y);
           const TileConf tc = pl.conf[pl.order[i]];
           const std::vector<TileGroup> one{TileGroup{tc, 0u, vt}};
-          CKR(run_bin(c, vd + i, 1, vt, cnt + i, capturing, one));
+          CKR(run_bin(c, vd + i, 1, vt, cnt + i, capturing, one, true, false));
           CKR(clear_moments(c, 1));
           CKR(need_targets());
           {
@@ -997,7 +1004,7 @@ int train_views(RmeshCtx* c, const RmeshCamera* cams, int n_views, const float* 
           CKR(run_sh_backward(c, vd + i, 1, capturing));
         }
       } else {
-        CKR(run_bin(c, vd, n_views, total_tiles, cnt, capturing, pl.groups));
+        CKR(run_bin(c, vd, n_views, total_tiles, cnt, capturing, pl.groups, true, build));
         CKR(clear_moments(c, n_views));
         CKR(need_targets());
         {
@@ -1499,9 +1506,10 @@ int rmesh_forward_views(RmeshCtx* c, const RmeshCamera* cams, int32_t n_views, f
     CKR(upload_views(c, n_views));
     Counters* cnt = c->counters_d.as<Counters>();
     CK(cudaMemsetAsync(cnt, 0, sizeof(Counters), c->stream));
-    CKR(run_records(c, false));
+    const bool build = n_views == 1;
+    if (!build) CKR(run_records(c, false));
     ViewParams* vd = c->views_d.as<ViewParams>();
-    CKR(run_bin(c, vd, n_views, total_tiles, cnt, false, pl.groups, false));
+    CKR(run_bin(c, vd, n_views, total_tiles, cnt, false, pl.groups, false, build));
     {
       StageScope sc(c, kStComposite, false);
       TileArgs ta = base_tile_args(c, vd, n_views, total_tiles, cnt);
@@ -1544,9 +1552,8 @@ int rmesh_forward_tiled(RmeshCtx* c, const RmeshCamera* cam, float* rgba_out, fl
     CKR(upload_views(c, 1));
     Counters* cnt = c->counters_d.as<Counters>();
     CK(cudaMemsetAsync(cnt, 0, sizeof(Counters), c->stream));
-    CKR(run_records(c, false));
     ViewParams* vd = c->views_d.as<ViewParams>();
-    CKR(run_bin(c, vd, 1, tiles, cnt, false, one));
+    CKR(run_bin(c, vd, 1, tiles, cnt, false, one, true, true));
     {
       StageScope sc(c, kStComposite, false);
       TileArgs ta = base_tile_args(c, vd, 1, tiles, cnt);

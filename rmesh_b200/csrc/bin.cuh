@@ -304,19 +304,30 @@ __global__ void __launch_bounds__(256) tile_order_hist_kernel(const uint2* __res
 // tiles in chunks of kOrderThreads: each tile's rank among the chunk's tiles
 // of its bucket comes from per-warp peer masks (one ballot per bucket bit)
 // and a per-bucket scan over the warps.
+// Up to kOrderSelfCount tiles the block counts the buckets itself (eight chunks
+// of reads cost less than another launch).
 constexpr int kOrderThreads = 1024;
+constexpr uint32_t kOrderSelfCount = 8 * kOrderThreads;
 __global__ void __launch_bounds__(kOrderThreads) tile_order_stable_kernel(const uint2* __restrict__ ranges,
                                                                           uint32_t n_tiles, const uint32_t* hist,
                                                                           uint32_t* order) {
   constexpr int kW = kOrderThreads / 32;
   __shared__ uint32_t cursor[kOrderBuckets];
   __shared__ uint32_t wcnt[kW][kOrderBuckets];
+  __shared__ uint32_t own[kOrderBuckets];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool self = n_tiles <= kOrderSelfCount;
+  if (tid < kOrderBuckets) own[tid] = self ? 0u : hist[tid];
+  __syncthreads();
+  if (self) {
+    for (uint32_t t = (uint32_t)tid; t < n_tiles; t += kOrderThreads) atomicAdd(&own[order_bucket(ranges[t])], 1u);
+    __syncthreads();
+  }
   if (tid == 0) {
     uint32_t acc = 0u;
     for (int b = kOrderBuckets - 1; b >= 0; --b) {
       cursor[b] = acc;
-      acc += hist[b];
+      acc += own[b];
     }
   }
   for (uint32_t base = 0; base < n_tiles; base += kOrderThreads) {

@@ -20,23 +20,37 @@ struct __align__(16) TetRec {
   float4 a, b, c, d;
 };
 
-__global__ void __launch_bounds__(256) build_records_kernel(int M, const float* __restrict__ verts,
-                                                            const uint4* __restrict__ idx4,
-                                                            const float* __restrict__ dens,
-                                                            const float* __restrict__ cgrad,
-                                                            const float* __restrict__ base,
-                                                            TetRec* __restrict__ rec, float4* __restrict__ color4) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= M) return;
-  uint4 q = idx4[t];
-  float g0 = cgrad[3 * t], g1 = cgrad[3 * t + 1], g2 = cgrad[3 * t + 2];
+// The mesh arrays a record is gathered from and where it goes.
+struct RecordArgs {
+  const float* verts;
+  const uint4* idx4;
+  const float* dens;
+  const float* cgrad;
+  const float* base;
+  TetRec* rec;
+  float4* color4;
+};
+
+__device__ __forceinline__ TetRec build_record(const RecordArgs& a, uint32_t t, float4& color) {
+  const uint4 q = a.idx4[t];
+  const float* v = a.verts;
+  const float g0 = a.cgrad[3 * (size_t)t], g1 = a.cgrad[3 * (size_t)t + 1], g2 = a.cgrad[3 * (size_t)t + 2];
   TetRec r;
-  r.a = make_float4(verts[3 * q.x], verts[3 * q.x + 1], verts[3 * q.x + 2], dens[t]);
-  r.b = make_float4(verts[3 * q.y], verts[3 * q.y + 1], verts[3 * q.y + 2], g0);
-  r.c = make_float4(verts[3 * q.z], verts[3 * q.z + 1], verts[3 * q.z + 2], g1);
-  r.d = make_float4(verts[3 * q.w], verts[3 * q.w + 1], verts[3 * q.w + 2], g2);
-  rec[t] = r;
-  if (color4) color4[t] = make_float4(base[3 * t], base[3 * t + 1], base[3 * t + 2], 0.0f);
+  r.a = make_float4(v[3 * (size_t)q.x], v[3 * (size_t)q.x + 1], v[3 * (size_t)q.x + 2], a.dens[t]);
+  r.b = make_float4(v[3 * (size_t)q.y], v[3 * (size_t)q.y + 1], v[3 * (size_t)q.y + 2], g0);
+  r.c = make_float4(v[3 * (size_t)q.z], v[3 * (size_t)q.z + 1], v[3 * (size_t)q.z + 2], g1);
+  r.d = make_float4(v[3 * (size_t)q.w], v[3 * (size_t)q.w + 1], v[3 * (size_t)q.w + 2], g2);
+  color = make_float4(a.base[3 * (size_t)t], a.base[3 * (size_t)t + 1], a.base[3 * (size_t)t + 2], 0.0f);
+  a.rec[t] = r;
+  a.color4[t] = color;
+  return r;
+}
+
+__global__ void __launch_bounds__(256) build_records_kernel(int M, RecordArgs a) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= M) return;
+  float4 color;
+  build_record(a, (uint32_t)t, color);
 }
 
 // Conservative scanline over tile rows (project_compute.wgsl:202-259 ==
@@ -284,13 +298,16 @@ struct ProjectArgs {
   int n_views;
   const ViewParams* views;
   const TetRec* rec;
+  // runs of one view: the records are gathered here (one launch fewer); otherwise
+  // build_records_kernel has written them
+  int build;
+  RecordArgs records;
   // per-item outputs at the item index i = tet * n_views + view (an entry's
   // index is its item index; items that touch no tile write only vis_cnt)
   uint32_t* vis_cnt;            // tiles_touched of a tile-touching item, 0 otherwise
   float4* vis_proj;             // 2 per entry: division-projected pixel coords (emission)
   TetView* vis_view;            // per entry: the tile kernel's per-(view, tet) record
-  const float4* color4;         // tet colours, [view * color_view_stride + tet]
-  uint32_t color_view_stride;
+  const float4* color4;         // tet colours
   // SH colours (sh != nullptr): coefficients [M][3][nc]; the colour of each
   // tile-touching entry goes to vis_color[i]
   const float* sh;
@@ -312,7 +329,8 @@ __global__ void __launch_bounds__(256, 3) project_kernel(ProjectArgs a) {
   const uint32_t tet = (uint32_t)(i / (unsigned long long)a.n_views);
   const uint32_t view = (uint32_t)(i - (unsigned long long)tet * a.n_views);
   const ViewParams& V = a.views[view];
-  const TetRec r = a.rec[tet];
+  float4 base_color = make_float4(0.f, 0.f, 0.f, 0.f);
+  const TetRec r = a.build ? build_record(a.records, tet, base_color) : a.rec[tet];
   const float vx[4] = {r.a.x, r.b.x, r.c.x, r.d.x};
   const float vy[4] = {r.a.y, r.b.y, r.c.y, r.d.y};
   const float vz[4] = {r.a.z, r.b.z, r.c.z, r.d.z};
@@ -382,7 +400,7 @@ __global__ void __launch_bounds__(256, 3) project_kernel(ProjectArgs a) {
       col = sh_color_deg(a.sh_degree, r, a.sh + (size_t)tet * 3 * nc, V.cam);
       a.vis_color[i] = col;
     } else {
-      col = a.color4[(size_t)a.color_view_stride * view + tet];
+      col = a.build ? base_color : a.color4[tet];
     }
     write_tet_view(a.vis_view + i, r, col, V);
   }

@@ -53,3 +53,18 @@ def test_both_sides_of_the_strip_rule(c1_scene, oracle32, size, threads):
     from rmesh_b200.camera import make_camera
 
     _check(c1_scene, oracle32, make_camera((2.1, -1.9, 0.9), (0.0, 0.0, 0.0), 50.0, size, size - 7), 12, threads)
+
+
+@pytest.mark.parametrize("n", [1, 4, 8, 16])
+def test_batched_views_equal_single_views(c1_scene, n):
+    """Batched runs split emission groups over 8, 4, 2 or 1 blocks, gather their
+    tet records in a kernel of their own (n > 1) and skip the adjoint's spans; each
+    image equals the single-view forward's bit for bit."""
+    from rmesh_b200.camera import orbit_cameras
+
+    cams = orbit_cameras(n, seed=5, radius=(2.2, 3.4), resolutions=((96, 80),))
+    r = make_renderer(c1_scene, cams[0])
+    imgs = r.forward_views(cams)
+    for c, img in zip(cams, imgs):
+        np.testing.assert_array_equal(img, r.forward_tiled(c.cam_pos, c.vp, c.c2w_intrinsics))
+    r.close()
