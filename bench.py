@@ -332,8 +332,8 @@ def run_gpu(args):
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 4),
                      "traffic": int(TILE_DRAM_BYTES_PER_PAIR * int(info.n_pairs_last)),
-                     "kernel": f"tile_kernel<{tile_size},kModeTrain> (fused forward+loss+adjoint, "
-                               f"{tile_threads} threads per tile)",
+                     "kernel": f"strip_kernel<{tile_size},kModeTrain> (fused forward+loss+adjoint, "
+                               f"one warp per strip of tile rows)",
                      "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else
                      "fallback 6.65 TB/s", "launch_ms": round(comp_ms, 4), "algorithmic_bytes": alg,
                      "n_pairs": int(info.n_pairs_last)},
@@ -626,8 +626,8 @@ def run_training(args):
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 4),
                      "traffic": int(TILE_DRAM_BYTES_PER_PAIR * int(info.n_pairs_last)),
-                     "kernel": f"tile_kernel<{tile[0]},kModeTrain> (fused forward+loss+adjoint, "
-                               f"{tile[1]} threads per tile)",
+                     "kernel": f"strip_kernel<{tile[0]},kModeTrain> (fused forward+loss+adjoint, "
+                               f"one warp per strip of tile rows)",
                      "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else
                      "fallback 6.65 TB/s", "launch_ms": round(comp_ms, 4), "algorithmic_bytes": alg,
                      "n_pairs": int(info.n_pairs_last)},

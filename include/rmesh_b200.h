@@ -98,7 +98,7 @@ typedef struct {
   int32_t reserved;
 } RmeshTrainOpts;
 
-#define RMESH_MODE_PLAIN 0    /* one launch sequence per view, one tile per CTA */
+#define RMESH_MODE_PLAIN 0    /* one launch sequence per view, one strip per warp */
 #define RMESH_MODE_BATCHED 1  /* all views in one launch sequence, persistent (view,tile) queue */
 #define RMESH_MODE_GRAPH 2    /* BATCHED, captured as a CUDA graph per step signature (up to 8 kept) and replayed */
 
@@ -236,10 +236,10 @@ RMESH_API int rmesh_grad_slots(RmeshCtx* ctx, float** device_ptr, uint64_t* n_fl
 
 /* Tile configurations (no reference counterpart; the reference fixes 12-pixel
  * tiles, lib.rs:442).  A configuration is a tile size (8, 12 or 16) and the
- * threads per tile: one per pixel rounded up to whole warps (64, 160, 256; pass
- * 0 for it) or twice that (128, 320, 512: the item-parallel phases of the tile
- * kernel get more threads and larger sub-batches, half as many tiles are
- * resident per SM).  The pair-sort key width follows from the tile count.
+ * threads per tile, which name how finely its work is split: one per pixel
+ * rounded up to whole warps (64, 160, 256; pass 0 for it) stands for strips of 4
+ * tile rows per warp (2 or 1 in small launches), twice that (128, 320, 512) for
+ * strips of half as many rows.  The pair-sort key width follows from the tile count.
  * set_tile_config sets the default configuration; set_resolution_tile_config
  * gives views of width x height their own (tile_size 0 removes it), so one
  * multi-view step can run, e.g., its 256x256 views at tile 8 and the rest at

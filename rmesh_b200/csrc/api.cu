@@ -798,9 +798,8 @@ int clear_moments(RmeshCtx* c, int n_views) {
   return RMESH_OK;
 }
 
-// the tets' gradients from an adjoint launch's moments
-int run_grad_finalize(RmeshCtx* c, int n_views, bool capturing) {
-  StageScope sc(c, kStComposite, capturing);
+// the tets' gradients from an adjoint launch's moments (inside its composite scope)
+int run_grad_finalize(RmeshCtx* c, int n_views) {
   GradFinalizeArgs ga;
   ga.M = (int)c->M;
   ga.n_views = n_views;
@@ -999,8 +998,8 @@ int train_views(RmeshCtx* c, const RmeshCamera* cams, int n_views, const float* 
             TileArgs ta = base_tile_args(c, vd + i, 1, vt, cnt + i);
             ta.gt_rgb = gt_dev;
             CKR((launch_tile_m<kModeTrain, false>(c, ta, vt, false, tc)));
+            CKR(run_grad_finalize(c, 1));
           }
-          CKR(run_grad_finalize(c, 1, capturing));
           CKR(run_sh_backward(c, vd + i, 1, capturing));
         }
       } else {
@@ -1012,8 +1011,8 @@ int train_views(RmeshCtx* c, const RmeshCamera* cams, int n_views, const float* 
           TileArgs ta = base_tile_args(c, vd, n_views, total_tiles, cnt);
           ta.gt_rgb = gt_dev;
           CKR((launch_groups<kModeTrain, false>(c, ta, pl.groups)));
+          CKR(run_grad_finalize(c, n_views));
         }
-        CKR(run_grad_finalize(c, n_views, capturing));
         CKR(run_sh_backward(c, vd, n_views, capturing));
       }
       if (do_adam) CKR(launch_adam(c, n_cnt, capturing));
@@ -1623,10 +1622,10 @@ static int backward_impl(RmeshCtx* c, const float* dl, const float* dl_aux, floa
     } else {
       CKR((launch_groups<kModeBackward, false>(c, ta, one)));
     }
+    CKR(run_grad_finalize(c, 1));
   }
   if (d_aux && with_aux)
     CK(cudaMemcpyAsync(d_aux, c->d_aux.p, (uint64_t)c->M * c->aux_dim * 4, cudaMemcpyDefault, c->stream));
-  CKR(run_grad_finalize(c, 1, false));
   CKR(run_sh_backward(c, vd, 1, false));
   const size_t N = (size_t)c->N, M = (size_t)c->M;
   CKR(ensure_buf(c, c->out_a, 3 * N * 4));

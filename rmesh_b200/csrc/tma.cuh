@@ -1,10 +1,6 @@
-// mbarrier + TMA bulk-copy helpers (sm_90+ PTX, used on sm_100a).
-//
-// Only the plain, CTA-local form of cp.async.bulk is used: global -> this
-// CTA's shared memory, completion counted on a local mbarrier; every copy
-// reads this GPU's own memory.  Sources are 16-byte aligned and sizes are multiples
-// of 16 bytes (144-byte per-view tet records, span-cache rows of 32/48/64
-// bytes per tet).
+// Asynchronous copies into shared memory, and the bounded mbarrier wait (sm_90+
+// PTX, used on sm_100a).  Every copy reads this GPU's own memory, 16 bytes at
+// 16-byte aligned addresses.
 #pragma once
 #include <stdint.h>
 
@@ -21,31 +17,6 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
 // Make barrier initialisation visible to the async proxy.
 __device__ __forceinline__ void fence_mbar_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-// Order this thread's earlier generic-proxy shared-memory accesses before
-// subsequent async-proxy (bulk copy) accesses.
-__device__ __forceinline__ void fence_proxy_async_smem() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
-// Order this thread's earlier generic-proxy global-memory writes before
-// later async-proxy (bulk copy) reads of them.
-__device__ __forceinline__ void fence_proxy_async_global() {
-  asm volatile("fence.proxy.async.global;" ::: "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-               : "memory");
-}
-
-__device__ __forceinline__ void bulk_copy_g2s(void* dst_smem, const void* src_gmem, uint32_t bytes, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-          smem_u32(dst_smem)),
-      "l"(src_gmem), "r"(bytes), "r"(smem_u32(bar))
-      : "memory");
 }
 
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
