@@ -47,26 +47,32 @@ RES = ((256, 256), (512, 512), (800, 600), (1024, 1024))
 N_VIEWS = 16
 LR = dict(lr_verts=1e-4, lr_dens=1e-2, lr_grads=1e-3)
 LR_SH = 2.5e-3
-# DRAM bytes (read + write) per (tile, tet) pair of the fused compositing
-# kernel, from a one-kernel ncu capture of a 4-view case of this workload's
-# mesh and resolution mix (bench.py --views 4: 8.13 M pairs,
-# dram__bytes_read.sum + dram__bytes_write.sum = 2.907 GB); the roofline's
-# "traffic" scales it to the run's pair count.
-TILE_DRAM_BYTES_PER_PAIR = 358.0
-# Warp instructions per (tile, tet) pair of the same kernel, from the same
-# capture (smsp__inst_executed.sum = 9.408 G); the issue ceiling is 148 SMs x
-# 4 schedulers x one instruction per clock.
-TILE_WARP_INST_PER_PAIR = 1157.0
+# Per (tile, tet) pair of the fused compositing kernel, by tile size: DRAM bytes
+# (dram__bytes_read.sum + dram__bytes_write.sum) and warp instructions
+# (smsp__inst_executed.sum), each from a one-pass ncu capture of this workload's
+# step (--profile-one-step --tile-size T: 38.33 M pairs at 12, 8.30 GB and 35.07 G;
+# 58.17 M pairs at 8, 7.93 GB and 31.71 G).  The issue ceiling is 148 SMs x 4
+# schedulers x one instruction per clock.  Sizes without a capture report null.
+TILE_DRAM_BYTES_PER_PAIR = {12: 216.6, 8: 136.4}
+TILE_WARP_INST_PER_PAIR = {12: 915.0, 8: 545.0}
 
 
-def issue_roofline(n_pairs: int, launch_ms: float, sm_mhz) -> dict:
+def dram_traffic(n_pairs: int, tile_size: int):
+    per_pair = TILE_DRAM_BYTES_PER_PAIR.get(tile_size)
+    return None if per_pair is None else int(per_pair * n_pairs)
+
+
+def issue_roofline(n_pairs: int, launch_ms: float, sm_mhz, tile_size: int):
     """The tile kernel's bound in practice: instruction issue, not HBM."""
+    per_pair = TILE_WARP_INST_PER_PAIR.get(tile_size)
+    if per_pair is None:
+        return None
     mhz = float(sm_mhz) if sm_mhz else 1965.0
     peak = 148 * 4 * mhz * 1e6 / 1e12
-    achieved = TILE_WARP_INST_PER_PAIR * n_pairs / (launch_ms * 1e-3) / 1e12
+    achieved = per_pair * n_pairs / (launch_ms * 1e-3) / 1e12
     return {"achieved": round(achieved, 4), "peak": round(peak, 4), "unit": "T warp-instructions/s",
             "frac": round(achieved / peak, 4),
-            "basis": f"{TILE_WARP_INST_PER_PAIR:.0f} warp instructions per pair (ncu) x pairs / launch time; "
+            "basis": f"{per_pair:.0f} warp instructions per pair (ncu) x pairs / launch time; "
                      f"peak 148 SMs x 4 schedulers x {mhz:.0f} MHz"}
 
 
@@ -331,13 +337,13 @@ def run_gpu(args):
         "stage_ms_per_step": {k: round(v / nsteps_prof, 4) for k, v in stage_ms.items()},
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 4),
-                     "traffic": int(TILE_DRAM_BYTES_PER_PAIR * int(info.n_pairs_last)),
+                     "traffic": dram_traffic(int(info.n_pairs_last), tile_size),
                      "kernel": f"strip_kernel<{tile_size},kModeTrain> (fused forward+loss+adjoint, "
                                f"one warp per strip of tile rows)",
                      "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else
                      "fallback 6.65 TB/s", "launch_ms": round(comp_ms, 4), "algorithmic_bytes": alg,
                      "n_pairs": int(info.n_pairs_last)},
-        "issue_roofline": issue_roofline(int(info.n_pairs_last), comp_ms, clocks.get("sm_mhz")),
+        "issue_roofline": issue_roofline(int(info.n_pairs_last), comp_ms, clocks.get("sm_mhz"), tile_size),
         "clocks": clocks,
     }
     if rank == 0 and not args.no_cpu_baseline:
@@ -625,13 +631,13 @@ def run_training(args):
         "stage_ms_per_step": {k: round(v / nb, 4) for k, v in stage_ms.items()},
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 4),
-                     "traffic": int(TILE_DRAM_BYTES_PER_PAIR * int(info.n_pairs_last)),
+                     "traffic": dram_traffic(int(info.n_pairs_last), tile[0]),
                      "kernel": f"strip_kernel<{tile[0]},kModeTrain> (fused forward+loss+adjoint, "
                                f"one warp per strip of tile rows)",
                      "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else
                      "fallback 6.65 TB/s", "launch_ms": round(comp_ms, 4), "algorithmic_bytes": alg,
                      "n_pairs": int(info.n_pairs_last)},
-        "issue_roofline": issue_roofline(int(info.n_pairs_last), comp_ms, clocks.get("sm_mhz")),
+        "issue_roofline": issue_roofline(int(info.n_pairs_last), comp_ms, clocks.get("sm_mhz"), tile[0]),
         "clocks": clocks,
         "training": {"lr_verts": lr["lr_verts"],
                      "loss_first_pass": fin(losses[:nb].mean()), "loss_last_pass": fin(losses[-nb:].mean()),
