@@ -90,6 +90,7 @@ struct RmeshCtx {
   // host targets of a step are copied on their own stream beside the binning
   cudaStream_t copy_stream = nullptr;
   cudaEvent_t copy_begin = nullptr, copy_done = nullptr;
+  bool host_targets_seen = false;
   int64_t N = 0, M = 0;
   int width = 0, height = 0, tile_size = 12;
   int tile_wide = 0;  // default tile configuration: tile_size, threads per tile doubled when set
@@ -955,8 +956,10 @@ int train_views(RmeshCtx* c, const RmeshCamera* cams, int n_views, const float* 
     const float* gt_dev = direct_gt ? gt : c->gt.as<float>();
     // host targets: a replayed graph needs them before its launch; otherwise they
     // are copied on a second stream once the binning that does not read them is
-    // enqueued (after work the caller ordered on the context's stream before)
-    const bool beside = !direct_gt && mode != RMESH_MODE_GRAPH;
+    // enqueued (after work the caller ordered on the context's stream before).  The
+    // context's first step copies in line: making the stream costs more than it hides.
+    const bool beside = !direct_gt && mode != RMESH_MODE_GRAPH && c->host_targets_seen;
+    if (!direct_gt) c->host_targets_seen = true;
     if (!direct_gt && !beside) CK(cudaMemcpyAsync(c->gt.p, gt, total_pix * 12, cudaMemcpyHostToDevice, c->stream));
     if (beside) {
       if (!c->copy_stream) {
