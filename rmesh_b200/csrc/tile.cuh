@@ -63,7 +63,7 @@ __device__ __forceinline__ uint8_t pack_span(short2 sp) {
 // (S, P.x, P.y, P.z) of face f, 16 density, 17..19 colour, 20 the sum of the three
 // colour gradients, 21..23 the colour gradient's gradient.
 constexpr int kMom = 24;
-// error statistics per tet: 11 sums and a maximum
+// error statistics per tet: 10 sums, then two integer words: the pixel count and a maximum
 constexpr int kErrMom = 12;
 // per-lane rows of the warp's reduction buffers, with strides that spread a column
 // of 16-byte accesses over all banks: the 16 face sums (column 16 free), and the
@@ -752,7 +752,8 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : (TS == 16 || MODE 
       }
     };
     // the same for the error statistics: lane c sums column c over each tet's
-    // adjacent rows, the last column (integers) by maximum
+    // adjacent rows; the last two columns are integers, a sum (exact at any image
+    // size) and a maximum
     auto combine_error = [&](int base, float* dst) {
       const int n_rows = min(32, n_runs - base);
       int k = rk0;
@@ -762,14 +763,21 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : (TS == 16 || MODE 
         const uint32_t entry = __shfl_sync(0xffffffffu, bv, k);
         if (lane < kErrMom) {
           float* at = dst + (size_t)entry * kErrMom + lane;
-          if (lane == kErrMom - 1) {
-            int mx = 0;
-            for (int r = r0; r < r1; ++r) mx = max(mx, __float_as_int(s.red[r][lane]));
-            if (mx > 0) atomicMax(reinterpret_cast<int*>(at), mx);
-          } else {
-            float sum = s.red[r0][lane];
-            for (int r = r0 + 1; r < r1; ++r) sum += s.red[r][lane];
+          float sum = 0.0f;
+          uint32_t count = 0u;
+          int mx = 0;
+          for (int r = r0; r < r1; ++r) {  // one walk for the three kinds of column
+            const float v = s.red[r][lane];
+            sum += v;
+            count += __float_as_uint(v);
+            mx = max(mx, __float_as_int(v));
+          }
+          if (lane < kErrMom - 2) {
             if (sum != 0.0f) atomicAdd(at, sum);
+          } else if (lane == kErrMom - 2) {
+            if (count != 0u) atomicAdd(reinterpret_cast<uint32_t*>(at), count);
+          } else {
+            if (mx > 0) atomicMax(reinterpret_cast<int*>(at), mx);
           }
         }
         r0 = r1;
@@ -945,7 +953,7 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : (TS == 16 || MODE 
           float acc[kErrMom];
 #pragma unroll
           for (int i = 0; i < kErrMom; ++i) acc[i] = 0.0f;
-          int mx = 0;
+          int count = 0, mx = 0;
           for (int j = 0, slot = lane * R; j < rlen; ++j, ++slot) {
             const float2 st = s.a.ex[slot];
             if (!(st.y > 0.5f)) continue;
@@ -961,9 +969,10 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : (TS == 16 || MODE 
             acc[3] += w * e.y;
             acc[4] += w * (ox + d.x * ix.x); acc[5] += w * (oy + d.y * ix.x); acc[6] += w * (oz + d.z * ix.x);
             acc[7] += w * (ox + d.x * ix.y); acc[8] += w * (oy + d.y * ix.y); acc[9] += w * (oz + d.z * ix.y);
-            acc[10] += 1.0f;
+            ++count;
             mx = max(mx, __float2int_rz(65535.0f * w));
           }
+          acc[10] = __int_as_float(count);
           acc[11] = __int_as_float(mx);
 #pragma unroll
           for (int i = 0; i < kErrMom; ++i) s.red[lane][i] = acc[i];
@@ -1422,12 +1431,13 @@ __global__ void __launch_bounds__(256) error_finalize_kernel(int M, const float*
   const TetRec r = rec[t];
   const float cx = (r.a.x + r.b.x + r.c.x + r.d.x) * 0.25f, cy = (r.a.y + r.b.y + r.c.y + r.d.y) * 0.25f,
               cz = (r.a.z + r.b.z + r.c.z + r.d.z) * 0.25f;
-  const bool some = c.z != 0.0f;
+  const int count = __float_as_int(c.z);
+  const bool some = count != 0;
   e[0] = make_float4(a.x, a.y, a.z, 0.0f);
   e[1] = make_float4(0.0f, a.w, b.x, b.y);
   e[2] = make_float4(b.z, b.w, c.x, c.y);
   e[3] = some ? make_float4(a.x, a.x * cx, a.x * cy, a.x * cz) : make_float4(0.f, 0.f, 0.f, 0.f);
-  tet_count[2 * (size_t)t] = (int)c.z;
+  tet_count[2 * (size_t)t] = count;
   tet_count[2 * (size_t)t + 1] = __float_as_int(c.w);
 }
 

@@ -39,6 +39,26 @@ def test_error_stats_match_oracle(c1_scene, oracle32, res, ts):
     assert rel_l2(err2, err) <= 1e-6 and np.array_equal(cnt2[:, 0], cnt[:, 0])
 
 
+def test_pixel_count_is_exact_above_2_to_24():
+    """One tet over every pixel of a 577x65535 image: its count is the image's
+    37,813,695 pixels.  The last tile column is one pixel wide, so strips there add 2
+    or 1, which a 32-bit float sum above 2^25 no longer takes up."""
+    from conftest import known_tet_scene
+
+    from rmesh_b200.camera import make_camera
+
+    w, h = 577, 65535
+    # 5 degrees: every ray meets the ball inside the tet (radius 0.28, seen under 11 degrees)
+    cam = make_camera((1.8, -2.1, 1.2), (0.0, 0.0, 0.0), 5.0, w, h)
+    r = make_renderer(known_tet_scene(), cam)
+    img = r.forward_tiled(cam.cam_pos, cam.vp, cam.c2w_intrinsics)
+    assert img[..., 3].min() > 0.1
+    ones = np.ones(w * h, np.float32)
+    err, cnt = r.forward_error(ones, ones)
+    assert cnt[0, 0] == w * h > 1 << 25
+    r.close()
+
+
 def test_error_requires_forward(c1_scene):
     from rmesh_b200 import RMeshError
 
