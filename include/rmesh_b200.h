@@ -167,14 +167,15 @@ RMESH_API int rmesh_set_lr_sh(RmeshCtx* ctx, float lr_sh);
 
 /* ---- the path ------------------------------------------------------------- */
 /* forward_tiled, lib.rs:1041-1204: project -> bin -> sort -> ranges -> composite.
- * rgba_out [H][W][4]; aux_out [H][W][8 + aux_dim] or NULL (render_aux). */
+ * rgba_out [H][W][4]; aux_out [H][W][8 + aux_dim] or NULL (render_aux).  A call
+ * that fails in its run (overflow, timeout) writes neither. */
 RMESH_API int rmesh_forward_tiled(RmeshCtx* ctx, const RmeshCamera* cam, float* rgba_out, float* aux_out);
 
 /* Batched forward (no reference counterpart; the forward half of
  * rmesh_train_step_views): n_views cameras of any sizes rendered by one
  * persistent launch.  rgba_out receives the views' [H][W][4] images back to
  * back, aux_out (optional) their [H][W][8 + aux_dim] aux images back to back.
- * Images equal rmesh_forward_tiled's per view.  rmesh_backward does not
+ * Images equal rmesh_forward_tiled's per view; a failing run writes nothing.  rmesh_backward does not
  * follow this call (it follows a single-view rmesh_forward_tiled). */
 RMESH_API int rmesh_forward_views(RmeshCtx* ctx, const RmeshCamera* cams, int32_t n_views, float* rgba_out,
                                   float* aux_out);
@@ -349,6 +350,9 @@ RMESH_API int rmesh_debug_tiles_touched(RmeshCtx* ctx, uint32_t* out);
 RMESH_API int rmesh_debug_pairs(RmeshCtx* ctx, uint32_t* tile_ids, uint32_t* tet_ids, uint64_t cap, uint64_t* n);
 /* [start, end) per tile of the last forward ([2 * tiles]). */
 RMESH_API int rmesh_debug_ranges(RmeshCtx* ctx, uint32_t* ranges, uint64_t n_tiles);
+/* Stops the growth of the context's (tile, tet) slots at limit (0: the default,
+ * 2^31 - 1), so that a run which needs more fails with RMESH_ERR_PAIR_OVERFLOW. */
+RMESH_API int rmesh_debug_limit_pairs(RmeshCtx* ctx, uint64_t limit);
 
 /* No reference counterpart: runs the path's two bounded waits (chained-scan
  * look-back, TMA mbarrier) on conditions that never resolve and returns, in

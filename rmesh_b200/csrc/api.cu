@@ -69,6 +69,9 @@ struct DevBuf {
   }
 };
 
+// (tile, tet) slots of a run at most: slot numbers are 31-bit in the sorts
+constexpr uint64_t kMaxPairs = (1ull << 31) - 1;
+
 enum Stage { kStRecords = 0, kStProject, kStTetSort, kStEmit, kStPairSort, kStRanges, kStComposite, kStAdam, kStShAdjoint };
 // NVTX range names of the stages (profilers can select kernels by them, e.g.
 // ncu --nvtx --nvtx-include "rmesh/composite/")
@@ -131,6 +134,7 @@ struct RmeshCtx {
   DevBuf tile_order;  // longest-first tile order of the run
   DevBuf err_in, err_out;  // per-pixel error inputs, per-tet error statistics
   uint64_t cap_pairs = 0;
+  uint64_t pair_limit = kMaxPairs;  // growth of the pair buffers stops here
   uint64_t generation = 0;  // bumped whenever a buffer is reallocated
 
   // pinned host staging
@@ -445,7 +449,7 @@ int ensure_run_buffers(RmeshCtx* c, int n_views, uint64_t total_pixels, uint32_t
   if (c->sh_degree >= 0) {
     CKR(ensure_buf(c, c->vis_color, items * 16));
   }
-  if (c->cap_pairs == 0) c->cap_pairs = std::max<uint64_t>(8 * items, 1u << 16);
+  if (c->cap_pairs == 0) c->cap_pairs = std::min(std::max<uint64_t>(8 * items, 1u << 16), c->pair_limit);
   CKR(ensure_buf(c, c->pair_key, c->cap_pairs * 4));
   CKR(ensure_buf(c, c->pair_val, c->cap_pairs * 4));
   CKR(ensure_buf(c, c->pair_key_alt, c->cap_pairs * 4));
@@ -839,15 +843,8 @@ int run_sh_backward(RmeshCtx* c, const ViewParams* views_dev, int n_views, bool 
   return RMESH_OK;
 }
 
-// Counters of a run: enqueue_counters orders their copy behind the run,
-// sync_counters waits for the stream (with whatever was enqueued since) and
-// evaluates them.
-int enqueue_counters(RmeshCtx* c, int n) {
+int sync_counters(RmeshCtx* c, int n) {
   CK(cudaMemcpyAsync(c->counters_h, c->counters_d.p, sizeof(Counters) * n, cudaMemcpyDeviceToHost, c->stream));
-  return RMESH_OK;
-}
-int sync_counters(RmeshCtx* c, int n, bool enqueued = false) {
-  if (!enqueued) CKR(enqueue_counters(c, n));
   CK(cudaStreamSynchronize(c->stream));
   uint32_t bits = 0;
   uint64_t nv = 0, np = 0;
@@ -865,9 +862,8 @@ int sync_counters(RmeshCtx* c, int n, bool enqueued = false) {
 // grows pair capacity after an overflow; returns true when a retry makes sense
 bool grow_pairs(RmeshCtx* c) {
   const uint64_t need = c->last_n_pairs + c->last_n_pairs / 4 + 4096;
-  const uint64_t limit = (1ull << 31) - 1;
-  if (need <= c->cap_pairs || c->cap_pairs >= limit) return false;
-  c->cap_pairs = std::min(need, limit);
+  if (need <= c->cap_pairs || c->cap_pairs >= c->pair_limit) return false;
+  c->cap_pairs = std::min(need, c->pair_limit);
   return true;
 }
 
@@ -1525,13 +1521,13 @@ int rmesh_forward_views(RmeshCtx* c, const RmeshCamera* cams, int32_t n_views, f
         CKR((launch_groups<kModeForward, false>(c, ta, pl.groups)));
       }
     }
-    // one wait for counters and images (an overflowed run writes them again)
-    CKR(enqueue_counters(c, 1));
-    CK(cudaMemcpyAsync(rgba_out, c->rgba.p, total_pix * 16, cudaMemcpyDefault, c->stream));
-    if (aux_out) CK(cudaMemcpyAsync(aux_out, c->aux.p, aux_floats * 4, cudaMemcpyDefault, c->stream));
-    CKR(sync_counters(c, 1, true));
+    // the caller's arrays are written by a run that succeeded, not before
+    CKR(sync_counters(c, 1));
     if ((c->last_err_bits & kErrPairOverflow) && grow_pairs(c)) continue;
     CKR(status_from_bits(c));
+    CK(cudaMemcpyAsync(rgba_out, c->rgba.p, total_pix * 16, cudaMemcpyDefault, c->stream));
+    if (aux_out) CK(cudaMemcpyAsync(aux_out, c->aux.p, aux_floats * 4, cudaMemcpyDefault, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
     c->have_forward = false;
     c->last_views = n_views;
     return RMESH_OK;
@@ -1569,13 +1565,13 @@ int rmesh_forward_tiled(RmeshCtx* c, const RmeshCamera* cam, float* rgba_out, fl
         CKR((launch_groups<kModeForward, false>(c, ta, one)));
       }
     }
-    // one wait for counters and image (an overflowed run writes it again)
-    CKR(enqueue_counters(c, 1));
-    CK(cudaMemcpyAsync(rgba_out, c->rgba.p, npix * 16, cudaMemcpyDefault, c->stream));
-    if (aux_out) CK(cudaMemcpyAsync(aux_out, c->aux.p, npix * (8 + (uint64_t)c->aux_dim) * 4, cudaMemcpyDefault, c->stream));
-    CKR(sync_counters(c, 1, true));
+    // the caller's arrays are written by a run that succeeded, not before
+    CKR(sync_counters(c, 1));
     if ((c->last_err_bits & kErrPairOverflow) && grow_pairs(c)) continue;
     CKR(status_from_bits(c));
+    CK(cudaMemcpyAsync(rgba_out, c->rgba.p, npix * 16, cudaMemcpyDefault, c->stream));
+    if (aux_out) CK(cudaMemcpyAsync(aux_out, c->aux.p, npix * (8 + (uint64_t)c->aux_dim) * 4, cudaMemcpyDefault, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
     c->have_forward = true;
     c->last_tiles = tiles;
     c->last_views = 1;
@@ -1911,6 +1907,14 @@ int rmesh_debug_pairs(RmeshCtx* c, uint32_t* tiles, uint32_t* tets, uint64_t cap
     CK(cudaMemcpyAsync(tets, scratch, k * 4, cudaMemcpyDefault, c->stream));
   }
   CK(cudaStreamSynchronize(c->stream));
+  return RMESH_OK;
+}
+
+int rmesh_debug_limit_pairs(RmeshCtx* c, uint64_t limit) {
+  if (!c) return RMESH_ERR_INVALID_ARG;
+  c->pair_limit = limit == 0 ? kMaxPairs : std::min(std::max<uint64_t>(limit, 256), kMaxPairs);
+  c->cap_pairs = std::min(c->cap_pairs, c->pair_limit);
+  c->have_forward = false;  // the last run's lists are laid out by the capacity
   return RMESH_OK;
 }
 

@@ -109,6 +109,53 @@ def test_pair_buffer_overflow_grows_and_retries(oracle32):
     r.close()
 
 
+@pytest.mark.parametrize("where", ["host", "device"])
+def test_failing_forward_writes_nothing(c1_scene, where):
+    """A view that needs more (tile, tet) slots than the context may hold fails; the
+    caller's image and aux arrays keep every byte, a backward pass is refused, and
+    the same calls succeed once the slots may grow."""
+    import torch
+
+    from conftest import c1_camera
+    from rmesh_b200 import RMeshError, _lib
+    from rmesh_b200.renderer import _camera_struct
+
+    cam = c1_camera(256, 256)
+    args = (cam.cam_pos, cam.vp, cam.c2w_intrinsics)
+    ref = make_renderer(c1_scene, cam)
+    want, want_aux = ref.forward_tiled(*args, render_aux=True)
+    assert ref.info().n_pairs_last > 4096
+    r = make_renderer(c1_scene, cam)
+    lib = _lib.load()
+    assert lib.rmesh_debug_limit_pairs(r._ctx, 4096) == _lib.RMESH_OK
+    dev = "cuda" if where == "device" else "cpu"
+    img = torch.full((2, 256, 256, 4), -7.0, device=dev)
+    aux = torch.full((256, 256, 8), -7.0, device=dev)
+
+    def views():
+        if where == "device":
+            return r.forward_views([cam, cam], out=img)
+        cams = (_lib.Camera * 2)(*[_camera_struct(*args, 256, 256)] * 2)
+        r._check(lib.rmesh_forward_views(r._ctx, cams, 2, img.data_ptr(), None))
+
+    for call in (lambda: r.forward_tiled_into(*args, img[0], aux), lambda: r.forward_tiled_into(*args, img[0]), views):
+        with pytest.raises(RMeshError) as e:
+            call()
+        assert e.value.code == _lib.RMESH_ERR_PAIR_OVERFLOW
+        assert bool((img == -7.0).all()) and bool((aux == -7.0).all())
+        with pytest.raises(RMeshError):
+            r.backward(want)
+    assert lib.rmesh_debug_limit_pairs(r._ctx, 0) == _lib.RMESH_OK
+    r.forward_tiled_into(*args, img[0], aux)
+    np.testing.assert_array_equal(img[0].cpu().numpy(), want)
+    np.testing.assert_array_equal(aux.cpu().numpy(), want_aux)
+    views()
+    for i in range(2):
+        np.testing.assert_array_equal(img[i].cpu().numpy(), want)
+    r.close()
+    ref.close()
+
+
 def test_long_tile_lists(c2_scene):
     """65k tets seen at 48x48 (16 tiles of 12x12): each tile's list holds
     thousands of tets (hundreds of 32-tet batches, each with its span records
