@@ -853,8 +853,9 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : (TS == 16 || MODE 
                 float enx = 0.f, eny = 0.f, enz = 0.f;
                 if (entry < 4) {
                   const float4 n = s.rec[k][entry];
-                  const float l = -rsqrtf(n.x * n.x + n.y * n.y + n.z * n.z);
-                  enx = n.x * l; eny = n.y * l; enz = n.z * l;
+                  // (the root and the quotients correctly rounded: an output of its own)
+                  const float l = sqrtf(n.x * n.x + n.y * n.y + n.z * n.z);
+                  enx = -n.x / l; eny = -n.y / l; enz = -n.z / l;
                 }
                 const float ta = Tj * alpha;
                 nd[q][0] += ta * enx; nd[q][1] += ta * eny; nd[q][2] += ta * enz;
