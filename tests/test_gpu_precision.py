@@ -14,6 +14,16 @@ UNIT = 2.0 ** -24
 FACES = ((0, 2, 1, 3), (1, 2, 3, 0), (0, 3, 2, 1), (3, 0, 1, 2))
 
 
+def _one_tet(v, density, color, grad):
+    from rmesh_b200.scenes import circumspheres
+
+    v = np.asarray(v, np.float32).ravel()
+    idx = np.arange(4, dtype=np.uint32)
+    return {"vertices": v, "indices": idx, "base_colors": np.asarray(color, np.float32),
+            "densities": np.array([density], np.float32), "color_grads": np.asarray(grad, np.float32),
+            "circumdata": circumspheres(v, idx)}
+
+
 def test_entry_normal_is_correctly_rounded():
     """2,000 opaque tets with integer vertices, so that the face normals are exact and
     the weight of a pixel inside one is exactly 1: the aux image holds the unit normal
@@ -51,3 +61,30 @@ def test_entry_normal_is_correctly_rounded():
     assert np.all(got[want == 0.0] == 0.0)
     err = np.abs(got - want)[want != 0.0] / np.abs(want[want != 0.0])
     assert err.max() <= 2.001 * UNIT
+
+
+def test_optical_depth_derivative_is_one_quotient():
+    """A tet crossed over exactly 2 units, its colour 1 at the entry and clipped to 0 at
+    the exit: the density's gradient is -2 dphi(od) and, at these depths, dphi = -1 / od^2
+    to the last bit.  Its errors are the rounding of od^2 (rms 0.4 units) and one fast
+    quotient's (0.4 were it correctly rounded); 0.8 together leaves that quotient 0.7."""
+    from rmesh_b200.camera import make_camera
+
+    v = ((-4, 0, -3), (4, 0, -3), (0, 0, 9), (0, 4, 3))
+    cam = make_camera((0.0, -4.0, 0.0), (0.0, 0.0, 0.0), 60.0, 1, 1)
+    r = make_renderer(_one_tet(v, 1.0, (1.0, 0.5, 0.5), (0.0, -1.0, 0.0)), cam)
+    p = r.get_params()
+    dl = np.array([[[1.0, 0.0, 0.0, 0.0]]], np.float32)
+    err = []
+    for d in np.random.default_rng(5).uniform(23.5, 43.5, 1500).astype(np.float32):
+        r.update_params(p["vertices"], p["base_colors"], np.array([d], np.float32), p["color_grads"])
+        r.forward_tiled(cam.cam_pos, cam.vp, cam.c2w_intrinsics)
+        g = r.backward(dl)["d_densities"][0]
+        od = 2.0 * float(d)
+        want = -2.0 * (np.exp(-od) * (od + 1.0) - 1.0) / od ** 2
+        err.append((float(g) - want) / want)
+    r.close()
+    err = np.array(err) / UNIT
+    # (__fdividef: two units in the last place, four of these)
+    assert np.abs(err).max() <= 1.0 + 4.0
+    assert np.sqrt((err ** 2).mean()) <= 0.8
