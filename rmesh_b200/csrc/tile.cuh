@@ -200,7 +200,10 @@ __device__ __forceinline__ bool intersect4(const float4* nrm, const float* num_o
 }
 
 // e^x and 1/x by the hardware approximations (one unit in the last place or
-// two; results and arguments below 2^-126 count as zero).
+// two; results and arguments below 2^-126 count as zero).  Where they are used,
+// that changes nothing: transmittances are compared with 1e-6, 1 - e^-od and the
+// series' sums round such an e^-od away, and 1/x of an x above 2^126 is 0 in
+// __fdividef too.
 __device__ __forceinline__ float exp_fast(float x) {
   float r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x * 1.4426950408889634f));
@@ -1131,7 +1134,9 @@ __global__ void __launch_bounds__(32 * kStripWarps, AUX ? 3 : (TS == 16 || MODE 
               if constexpr (AUX && MODE == kModeBackward) {
                 // the aux channels' own terms: d od += T_prev alpha_t aux_s (d alpha / d od =
                 // alpha_t); d a[tet][ai] += dl_aux[pixel][ai] T_prev alpha, below
-                d_od_aux = t_prev * I.alpha_t * s.aux[slot].x;
+                // (__expf: this is the one use of exp(-od) to which values below 2^-126,
+                // od > 87.3, can matter)
+                d_od_aux = t_prev * __expf(-I.od) * s.aux[slot].x;
                 s.aux[slot].y = t_prev * (1.0f - I.alpha_t);
               }
               const float d_od = clipf(d_od_state + d_od_int + d_od_aux, kMinVal, kMaxVal);

@@ -88,3 +88,24 @@ def test_optical_depth_derivative_is_one_quotient():
     # (__fdividef: two units in the last place, four of these)
     assert np.abs(err).max() <= 1.0 + 4.0
     assert np.sqrt((err ** 2).mean()) <= 0.8
+
+
+def test_aux_gradient_of_an_almost_opaque_tet():
+    """At od 87.4..87.9 alpha's derivative e^-od is below 2^-126, the smallest normal
+    number, and still the whole of the density's gradient when only an aux channel has
+    a loss.  e^-od rounds the exponent od log2(e), about 126, to 2^-18."""
+    from rmesh_b200 import RMeshRenderer
+    from rmesh_b200.camera import make_camera
+
+    v = ((-4, 0, -3), (4, 0, -3), (0, 0, 9), (0, 4, 3))
+    cam = make_camera((0.0, -4.0, 0.0), (0.0, 0.0, 0.0), 60.0, 1, 1)
+    for d in (43.7, 43.8, 43.95):
+        sc = _one_tet(v, d, (1.0, 0.5, 0.5), (0.0, 0.0, 0.0))
+        r = RMeshRenderer(sc["vertices"], sc["indices"], sc["base_colors"], sc["densities"], sc["color_grads"],
+                          sc["circumdata"], 1, 1, 1)
+        r.set_aux_data(np.ones(1, np.float32))
+        r.forward_tiled(cam.cam_pos, cam.vp, cam.c2w_intrinsics, render_aux=True)
+        g = r.backward(np.zeros((1, 1, 4), np.float32), np.full((1, 1, 1), 1e30, np.float32))
+        r.close()
+        want = 2.0 * np.exp(-2.0 * float(np.float32(d))) * 1e30
+        np.testing.assert_allclose(g["d_densities"][0], want, rtol=4 * 2.0 ** -18)
