@@ -28,6 +28,7 @@
 #include "project.cuh"
 #include "rmesh_file.cuh"
 #include "sh.cuh"
+#include "side_copy.h"
 #include "sort.cuh"
 #include "tile.cuh"
 
@@ -84,16 +85,30 @@ struct EventPair {
   cudaEvent_t a, b;
 };
 
+// SideCopy's calls
+struct CudaCopyApi {
+  using Error = cudaError_t;
+  using Stream = cudaStream_t;
+  using Event = cudaEvent_t;
+  static Error create_stream(Stream* s) { return cudaStreamCreateWithFlags(s, cudaStreamNonBlocking); }
+  static Error create_event(Event* e) { return cudaEventCreateWithFlags(e, cudaEventDisableTiming); }
+  static Error record(Event e, Stream s) { return cudaEventRecord(e, s); }
+  static Error wait(Stream s, Event e) { return cudaStreamWaitEvent(s, e, 0); }
+  static Error copy(void* dst, const void* src, size_t n, Stream s) {
+    return cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, s);
+  }
+  static void synchronize(Stream s) { cudaStreamSynchronize(s); }
+  static void destroy_event(Event e) { cudaEventDestroy(e); }
+  static void destroy_stream(Stream s) { cudaStreamDestroy(s); }
+};
+
 }  // namespace
 
 struct RmeshCtx {
   int device = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
-  // host targets of a step are copied on their own stream beside the binning
-  cudaStream_t copy_stream = nullptr;
-  cudaEvent_t copy_begin = nullptr, copy_done = nullptr;
-  bool host_targets_seen = false;
+  SideCopy<CudaCopyApi> targets;  // host targets of a step, copied beside the binning
   int64_t N = 0, M = 0;
   int width = 0, height = 0, tile_size = 12;
   int tile_wide = 0;  // default tile configuration: tile_size, threads per tile doubled when set
@@ -931,11 +946,22 @@ int train_views(RmeshCtx* c, const RmeshCamera* cams, int n_views, const float* 
   const uint32_t total_tiles = pl.total_tiles, max_tiles = pl.max_tiles;
   const int run_views = plain ? 1 : n_views;
   const bool direct_gt = is_device_ptr(gt);
+  // a step that fails returns with no copy of host targets under way
+  struct Settle {
+    RmeshCtx* c;
+    bool pending;
+    ~Settle() {
+      if (!pending) return;
+      cudaStreamSynchronize(c->stream);
+      c->targets.settle();
+    }
+  } settle{c, false};
   for (int attempt = 0; attempt < 4; ++attempt) {
     c->have_forward = false;  // the run's buffers may move
     CKR(ensure_run_buffers(c, run_views, total_pix, plain ? max_tiles : total_tiles));
     CKR(ensure_moments(c, run_views));
     if (!direct_gt) CKR(ensure_buf(c, c->gt, total_pix * 12));
+    settle.pending = !direct_gt;
     AdamParams& hp = *c->hp_h;
     hp.step = c->step + 1;
     hp.lr_verts = o->lr_verts;
@@ -952,27 +978,18 @@ int train_views(RmeshCtx* c, const RmeshCamera* cams, int n_views, const float* 
     const float* gt_dev = direct_gt ? gt : c->gt.as<float>();
     // host targets: a replayed graph needs them before its launch; otherwise they
     // are copied on a second stream once the binning that does not read them is
-    // enqueued (after work the caller ordered on the context's stream before).  The
-    // context's first step copies in line: making the stream costs more than it hides.
-    const bool beside = !direct_gt && mode != RMESH_MODE_GRAPH && c->host_targets_seen;
-    if (!direct_gt) c->host_targets_seen = true;
+    // enqueued (after work the caller ordered on the context's stream before)
+    const bool beside = !direct_gt && mode != RMESH_MODE_GRAPH;
     if (!direct_gt && !beside) CK(cudaMemcpyAsync(c->gt.p, gt, total_pix * 12, cudaMemcpyHostToDevice, c->stream));
     if (beside) {
-      if (!c->copy_stream) {
-        CK(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
-        CK(cudaEventCreateWithFlags(&c->copy_begin, cudaEventDisableTiming));
-        CK(cudaEventCreateWithFlags(&c->copy_done, cudaEventDisableTiming));
-      }
-      CK(cudaEventRecord(c->copy_begin, c->stream));
-      CK(cudaStreamWaitEvent(c->copy_stream, c->copy_begin, 0));
+      CK(c->targets.open());
+      CK(c->targets.follow(c->stream));
     }
     bool copied = false;
     auto need_targets = [&]() -> int {
       if (!beside || copied) return RMESH_OK;
       copied = true;
-      CK(cudaMemcpyAsync(c->gt.p, gt, total_pix * 12, cudaMemcpyHostToDevice, c->copy_stream));
-      CK(cudaEventRecord(c->copy_done, c->copy_stream));
-      CK(cudaStreamWaitEvent(c->stream, c->copy_done, 0));
+      CK(c->targets.copy(c->gt.p, gt, total_pix * 12, c->stream));
       return RMESH_OK;
     };
 
@@ -1068,6 +1085,8 @@ int train_views(RmeshCtx* c, const RmeshCamera* cams, int n_views, const float* 
       CKR(enqueue(false));
     }
     CKR(sync_counters(c, n_cnt));
+    settle.pending = false;  // waited for
+    c->targets.landed();
     if ((c->last_err_bits & kErrPairOverflow) && grow_pairs(c)) continue;
     CKR(status_from_bits(c));
     if (do_adam) c->step += 1;
@@ -1270,9 +1289,7 @@ int rmesh_destroy(RmeshCtx* c) {
     cudaEventDestroy(e.b);
   }
   for (auto e : c->event_pool) cudaEventDestroy(e);
-  if (c->copy_begin) cudaEventDestroy(c->copy_begin);
-  if (c->copy_done) cudaEventDestroy(c->copy_done);
-  if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
+  c->targets.close();
   if (c->views_h) cudaFreeHost(c->views_h);
   if (c->counters_h) cudaFreeHost(c->counters_h);
   if (c->hp_h) cudaFreeHost(c->hp_h);
