@@ -741,12 +741,16 @@ int launch_tile_t(RmeshCtx* c, TileArgs& ta, uint32_t n_tiles, bool persistent) 
 //   forward            0.6: 0.106 / 0.066 / 0.050 ms   8.1: 0.432 / 0.402 / 0.544 ms
 //                      45: 3.18 / 3.13 / 4.47 ms
 // The forward has little set-up and never gains from the four rows.  A wide
-// configuration (twice the threads per tile) takes one step thinner.
+// configuration (twice the threads per tile) takes two rows where the plain one takes
+// four; thinner than that it only lost (20,000 points at 1024x1024, one row instead of
+// two with 8- / 12-pixel tiles: forward call 1.70 / 1.38 against 1.15 / 0.96 ms, error
+// statistics 4.19 / 3.51 against 2.43 / 2.21; at 512x512 the fused step 1.43 / 1.27
+// against 0.96 / 0.93).
 int strip_rows(const RmeshCtx* c, uint32_t n_tiles, TileConf tc, bool adjoint) {
   const uint64_t strips4 = (uint64_t)n_tiles * (uint64_t)(tc.ts / 4);
   const uint64_t warps = (uint64_t)c->num_sms * 16u;
   const int rows = strips4 < warps ? 1 : (!adjoint || strips4 < 6 * warps ? 2 : 4);
-  return tc.wide ? std::max(1, rows / 2) : rows;
+  return tc.wide ? std::min(rows, 2) : rows;
 }
 
 template <int TS, int MODE, bool AUX>
