@@ -1762,7 +1762,39 @@ int time_views(RmeshCtx* c, const RmeshCamera* cams, int n, const float* gt, con
   CK(cudaEventRecord(e1, c->stream));
   CK(cudaEventSynchronize(e1));
   CK(cudaEventElapsedTime(ms, e0, e1));
-  *ms = std::rint(*ms * 500.0f) / 1000.0f;  // the mean of two, in whole microseconds (ties go to the earlier configuration)
+  *ms *= 0.5f;
+  return RMESH_OK;
+}
+
+// Times are compared in whole microseconds, ties to the earlier configuration:
+// smaller differences are not repeatable, and callers print them so.
+double whole_us(float ms) { return std::rint(1000.0 * (double)ms); }
+
+// A wide configuration runs other kernels than the plain one of its tile size only
+// where strip_rows says so; elsewhere the autotuner takes the plain one's time.
+bool wide_differs(RmeshCtx* c, const RmeshCamera* cams, int n, int ts) {
+  uint64_t tiles = 0;
+  for (int v = 0; v < n; ++v)
+    tiles += (uint64_t)((cams[v].width + ts - 1) / ts) * (uint64_t)((cams[v].height + ts - 1) / ts);
+  return strip_rows(c, (uint32_t)tiles, TileConf{ts, 0}, true) != strip_rows(c, (uint32_t)tiles, TileConf{ts, 1}, true);
+}
+
+// ms of each configuration of the grid on these views, and the best one
+int time_grid(RmeshCtx* c, const RmeshCamera* cams, int n, const float* gt, const RmeshTrainOpts& o, cudaEvent_t e0,
+              cudaEvent_t e1, const std::vector<TileConf>& grid, int w, int h, std::vector<RmeshTuneEntry>& out,
+              TileConf* best, float* best_ms) {
+  float ms = 0.f;
+  for (size_t i = 0; i < grid.size(); ++i) {
+    c->tile_size = grid[i].ts;
+    c->tile_wide = grid[i].wide;
+    // (the plain configuration of a tile size comes right before the wide one)
+    if (!grid[i].wide || wide_differs(c, cams, n, grid[i].ts)) CKR(time_views(c, cams, n, gt, o, e0, e1, &ms));
+    out.push_back(RmeshTuneEntry{w, h, grid[i].ts, conf_threads(grid[i]), ms});
+    if (i == 0 || whole_us(ms) < whole_us(*best_ms)) {
+      *best_ms = ms;
+      *best = grid[i];
+    }
+  }
   return RMESH_OK;
 }
 
@@ -1787,17 +1819,7 @@ int autotune_impl(RmeshCtx* c, const RmeshCamera* cams, int32_t n_views, const f
   // every configuration on all views
   TileConf best{c->tile_size, c->tile_wide};
   float best_ms = 0.f;
-  for (size_t i = 0; i < grid.size(); ++i) {
-    c->tile_size = grid[i].ts;
-    c->tile_wide = grid[i].wide;
-    float ms = 0.f;
-    CKR(time_views(c, cams, n_views, gt, o, e0, e1, &ms));
-    out.push_back(RmeshTuneEntry{0, 0, grid[i].ts, conf_threads(grid[i]), ms});
-    if (i == 0 || ms < best_ms) {
-      best_ms = ms;
-      best = grid[i];
-    }
-  }
+  CKR(time_grid(c, cams, n_views, gt, o, e0, e1, grid, 0, 0, out, &best, &best_ms));
   c->tile_size = best.ts;
   c->tile_wide = best.wide;
   // every configuration on the views of each resolution; a resolution whose
@@ -1816,17 +1838,7 @@ int autotune_impl(RmeshCtx* c, const RmeshCamera* cams, int32_t n_views, const f
       if (cams[v].width == r.first && cams[v].height == r.second) sub.push_back(cams[v]);
     TileConf rb = best;
     float rb_ms = 0.f;
-    for (size_t i = 0; i < grid.size(); ++i) {
-      c->tile_size = grid[i].ts;
-      c->tile_wide = grid[i].wide;
-      float ms = 0.f;
-      CKR(time_views(c, sub.data(), (int)sub.size(), gt, o, e0, e1, &ms));
-      out.push_back(RmeshTuneEntry{r.first, r.second, grid[i].ts, conf_threads(grid[i]), ms});
-      if (i == 0 || ms < rb_ms) {
-        rb_ms = ms;
-        rb = grid[i];
-      }
-    }
+    CKR(time_grid(c, sub.data(), (int)sub.size(), gt, o, e0, e1, grid, r.first, r.second, out, &rb, &rb_ms));
     if (!(rb == best)) chosen.push_back(RmeshCtx::ResConf{r.first, r.second, rb.ts, rb.wide});
   }
   c->tile_size = best.ts;
@@ -1836,7 +1848,7 @@ int autotune_impl(RmeshCtx* c, const RmeshCamera* cams, int32_t n_views, const f
   float mixed_ms = 0.f;
   CKR(time_views(c, cams, n_views, gt, o, e0, e1, &mixed_ms));
   out.push_back(RmeshTuneEntry{-1, -1, 0, 0, mixed_ms});
-  if (mixed_ms >= best_ms) c->res_conf.clear();
+  if (whole_us(mixed_ms) >= whole_us(best_ms)) c->res_conf.clear();
   return RMESH_OK;
 }
 

@@ -108,3 +108,32 @@ def test_grid_autotune(c1_scene):
     losses = r.train_step_views(cams, gts, 1e-4, 1e-2, 1e-3, 1, mode="graph")
     assert np.all(np.isfinite(losses)) and r.step == 1
     r.close()
+
+
+def test_autotune_times_a_kernel_once(c1_scene):
+    """Where a wide configuration launches the plain one's kernels (launches too small
+    for four-row strips), the grid gives it the plain one's time, and the timings are
+    the events', not rounded."""
+    import ctypes
+
+    from rmesh_b200 import _lib
+
+    cams, gts = _mixed_views()
+    r = make_renderer(c1_scene, cams[0])
+    n, cs, keep, p, o = r._views_args(cams, gts, 0.0, 0.0, 0.0, 1, 0.0, "batched")
+    entries = (_lib.TuneEntry * 64)()
+    got = ctypes.c_int32(0)
+    fine = False
+    for _ in range(8):
+        assert r._lib.rmesh_autotune(r._ctx, cs, n, p, ctypes.byref(o), 1, entries, 64, ctypes.byref(got)) == _lib.RMESH_OK
+        ms = {(e.width, e.height, e.tile_size, e.threads): e.ms for e in entries[:got.value] if e.width >= 0}
+        assert len(ms) == 4 * len(CONFIGS)
+        for (w, h, ts, th), t in ms.items():
+            plain = ((ts * ts + 31) // 32) * 32
+            assert t == ms[(w, h, ts, plain)]
+            fine = fine or abs(1000.0 * t - round(1000.0 * t)) > 0.05
+        assert r.tile_config()[1] in (64, 160, 256)
+        for c in cams:
+            assert r.tile_config(c.width, c.height)[1] in (64, 160, 256)
+    assert fine
+    r.close()
