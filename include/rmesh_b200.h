@@ -239,8 +239,10 @@ RMESH_API int rmesh_grad_slots(RmeshCtx* ctx, float** device_ptr, uint64_t* n_fl
  * tiles, lib.rs:442).  A configuration is a tile size (8, 12 or 16) and the
  * threads per tile, which name how finely its work is split: one per pixel
  * rounded up to whole warps (64, 160, 256; pass 0 for it) stands for strips of 4
- * tile rows per warp (2 or 1 in small launches), twice that (128, 320, 512) for
- * strips of half as many rows.  The pair-sort key width follows from the tile count.
+ * tile rows per warp in large launches with an adjoint (training steps, backward)
+ * and of 2, or in the smallest launches 1, elsewhere; twice that (128, 320, 512)
+ * for strips of 2 rows where the former takes 4, and otherwise the same.  The
+ * pair-sort key width follows from the tile count.
  * set_tile_config sets the default configuration; set_resolution_tile_config
  * gives views of width x height their own (tile_size 0 removes it), so one
  * multi-view step can run, e.g., its 256x256 views at tile 8 and the rest at

@@ -731,10 +731,9 @@ int launch_tile_t(RmeshCtx* c, TileArgs& ta, uint32_t n_tiles, bool persistent) 
 }
 
 // Rows per strip (4, 2 or 1) of a launch.  A strip is one warp's serial work, so
-// small launches take thinner strips until the chip has a few strips per
-// resident warp; thin strips repeat the per-tet set-up more often and fill fewer
-// pixel lanes.  Measured with 12-pixel tiles (tile kernel, 4 / 2 / 1 rows, in
-// units of 4-row strips per resident warp):
+// small launches take thinner strips until the chip has enough of them; thin strips
+// repeat the per-tet set-up more often and fill fewer pixel lanes.  Measured with
+// 12-pixel tiles (tile kernel, 4 / 2 / 1 rows, in units of 16 four-row strips per SM):
 //   forward + adjoint  2.3: 0.351 / 0.263 / 0.326 ms   2.5: 1.18 / 0.64 / 0.67 ms
 //                      4.3: 0.843 / 0.784 / 1.056 ms   9.4: 2.28 / 2.48 / 3.33 ms
 //                      79: 32.0 / 35.1 / 46.9 ms
@@ -755,11 +754,13 @@ int strip_rows(const RmeshCtx* c, uint32_t n_tiles, TileConf tc, bool adjoint) {
 
 template <int TS, int MODE, bool AUX>
 int launch_tile_s(RmeshCtx* c, TileArgs& ta, uint32_t n_tiles, bool persistent, TileConf tc) {
-  switch (strip_rows(c, n_tiles, tc, MODE == kModeBackward || MODE == kModeTrain)) {
-    case 1: return launch_tile_t<TS, 1, MODE, AUX>(c, ta, n_tiles, persistent);
-    case 2: return launch_tile_t<TS, 2, MODE, AUX>(c, ta, n_tiles, persistent);
-    default: return launch_tile_t<TS, 4, MODE, AUX>(c, ta, n_tiles, persistent);
+  constexpr bool kAdjoint = MODE == kModeBackward || MODE == kModeTrain;
+  const int rows = strip_rows(c, n_tiles, tc, kAdjoint);
+  if (rows == 1) return launch_tile_t<TS, 1, MODE, AUX>(c, ta, n_tiles, persistent);
+  if constexpr (kAdjoint) {  // the only launches of four rows
+    if (rows == 4) return launch_tile_t<TS, 4, MODE, AUX>(c, ta, n_tiles, persistent);
   }
+  return launch_tile_t<TS, 2, MODE, AUX>(c, ta, n_tiles, persistent);
 }
 
 // one launch over the tiles of a group (ta.tile_lo, ta.ticket set by the caller)
