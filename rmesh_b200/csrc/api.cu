@@ -451,6 +451,15 @@ struct RunState {
   }
 };
 
+// Status words of a sort of up to n keys.  New memory is cleared: a word left there by
+// another context's sort of the same epoch would count as published.
+int ensure_sort_status(RmeshCtx* c, uint64_t n) {
+  const size_t had = c->sort_status.bytes;
+  CKR(ensure_buf(c, c->sort_status, ((n + kSortPart - 1) / kSortPart + 1) * 256 * 8));
+  if (c->sort_status.bytes != had) CK(cudaMemsetAsync(c->sort_status.p, 0, c->sort_status.bytes, c->stream));
+  return RMESH_OK;
+}
+
 int ensure_run_buffers(RmeshCtx* c, int n_views, uint64_t total_pixels, uint32_t total_tiles) {
   const uint64_t items = (uint64_t)n_views * (uint64_t)c->M;
   CKR(ensure_buf(c, c->vis_key, items * 8));
@@ -471,8 +480,7 @@ int ensure_run_buffers(RmeshCtx* c, int n_views, uint64_t total_pixels, uint32_t
   CKR(ensure_buf(c, c->pair_val_alt, c->cap_pairs * 4));
   CKR(ensure_buf(c, c->spans_fwd, c->cap_pairs * 4 * kSpanWords));
   CKR(ensure_buf(c, c->spans_adj, c->cap_pairs * 4 * kSpanWords));
-  const uint64_t sort_items = std::max<uint64_t>(std::max<uint64_t>(items, c->cap_pairs), 4ull * c->M);
-  CKR(ensure_buf(c, c->sort_status, ((sort_items + kSortPart - 1) / kSortPart + 1) * 256 * 8));
+  CKR(ensure_sort_status(c, std::max<uint64_t>(std::max<uint64_t>(items, c->cap_pairs), 4ull * c->M)));
   CKR(ensure_buf(c, c->run_state, RunState(items, total_tiles).bytes));
   CKR(ensure_buf(c, c->tile_order, (uint64_t)std::max<uint32_t>(total_tiles, 1) * 4));
   CKR(ensure_buf(c, c->rgba, std::max<uint64_t>(total_pixels, 1) * 16));
@@ -1126,7 +1134,7 @@ int build_csr(RmeshCtx* c) {
   csr_fill_kernel<<<(unsigned)((n_refs + 255) / 256), 256, 0, c->stream>>>((int)c->M, c->idx.as<uint32_t>(),
                                                                           k0.as<uint32_t>(), c->csr_ref.as<uint32_t>());
   CKL();
-  CKR(ensure_buf(c, c->sort_status, ((n_refs + kSortPart - 1) / kSortPart + 1) * 256 * 8));
+  CKR(ensure_sort_status(c, n_refs));
   CK(cudaMemsetAsync(c->counters_d.p, 0, sizeof(Counters), c->stream));
   uint32_t* ok_keys = nullptr;
   uint32_t* ok_vals = nullptr;

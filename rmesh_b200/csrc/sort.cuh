@@ -3,17 +3,18 @@
 // Replaces the reference's 3-kernel-per-pass DeviceRadixSort
 // (crates/rmesh-sort/src/drs.rs:180-279, wgsl/drs_{upsweep,scan,downsweep}.wgsl):
 // one histogram kernel computes the digit counts of every pass in a single
-// read of the keys (each partition scans its pass's 256 counts itself), then each pass is ONE kernel that ranks a 4096-key
-// partition in shared memory (warp multi-split: peers of a digit found by one
-// ballot per digit bit), looks back
-// across earlier partitions for the per-digit global offset, and scatters
-// through shared memory so the writes are digit-contiguous.
+// read of the keys, then each pass is ONE kernel that ranks a 4096-key partition
+// in shared memory (warp multi-split: peers of a digit found by one ballot per
+// digit bit), looks back across earlier partitions for the per-digit offset (each
+// partition scans the pass's 256 counts itself), and scatters through shared
+// memory so the writes are digit-contiguous.
 //
 // Partitions are numbered by an atomic ticket, so every partition a block
 // waits on was started earlier (forward progress without co-residency).
 // Status words carry a device-side epoch instead of being cleared, so a
-// captured CUDA graph can replay the sort without memsets.  All spins are
-// bounded and raise kErrSpinTimeout instead of hanging.
+// captured CUDA graph can replay the sort without memsets; they start as zero (no
+// sort has epoch 0).  All spins are bounded and raise kErrSpinTimeout instead of
+// hanging.
 #pragma once
 #include "common.cuh"
 

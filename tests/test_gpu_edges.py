@@ -109,6 +109,25 @@ def test_pair_buffer_overflow_grows_and_retries(oracle32):
     r.close()
 
 
+def test_contexts_that_inherit_memory(c1_scene, oracle32):
+    """A view of at most 255 tiles sorts its pairs in one pass of several partitions.
+    Contexts made one after another get each other's freed memory, with the status
+    words of sorts that had the same numbers; each view's sorted pairs are the oracle's
+    all the same."""
+    from rmesh_b200.camera import orbit_cameras
+
+    for cam in orbit_cameras(6, seed=14, radius=(2.2, 3.0), resolutions=((180, 170),)):
+        ref = oracle32.forward_tiled(c1_scene, cam)
+        for _ in range(3):
+            r = make_renderer(c1_scene, cam)
+            r.forward_tiled(cam.cam_pos, cam.vp, cam.c2w_intrinsics)
+            assert r.info().n_pairs_last > 3 * 6144
+            tiles, tets = r.debug_pairs()
+            np.testing.assert_array_equal(tiles, ref["key_hi"])
+            np.testing.assert_array_equal(tets, ref["vals"])
+            r.close()
+
+
 @pytest.mark.parametrize("where", ["host", "device"])
 def test_failing_forward_writes_nothing(c1_scene, where):
     """A view that needs more (tile, tet) slots than the context may hold fails; the
