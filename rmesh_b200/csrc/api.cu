@@ -15,6 +15,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <initializer_list>
 #include <mutex>
 #include <cstdio>
 #include <cstring>
@@ -41,14 +42,22 @@ namespace {
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
+  bool part = false;  // of another buffer's allocation (place)
   DevBuf() = default;
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
   ~DevBuf() { release(); }
   void release() {
-    if (p) cudaFree(p);
+    if (p && !part) cudaFree(p);
     p = nullptr;
     bytes = 0;
+    part = false;
+  }
+  void place(void* at, size_t n) {
+    release();
+    p = at;
+    bytes = n;
+    part = true;
   }
   // grows (never shrinks); returns a cudaError_t; *grew set when reallocated
   cudaError_t ensure(size_t n, bool* grew = nullptr) {
@@ -108,6 +117,10 @@ struct RmeshCtx {
   int device = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
+  // allocations that the buffers below are parts of: the scene's, and the runs' by
+  // what their sizes follow (items, pairs, tiles and pixels)
+  DevBuf scene_mem, item_mem, pair_mem, tile_mem;
+  void* host_mem = nullptr;  // pinned: views_h, counters_h, hp_h
   SideCopy<CudaCopyApi> targets;  // host targets of a step, copied beside the binning
   int64_t N = 0, M = 0;
   int width = 0, height = 0, tile_size = 12;
@@ -331,6 +344,43 @@ int ensure_buf(RmeshCtx* c, DevBuf& b, size_t bytes) {
     if (r__ != RMESH_OK) return r__; \
   } while (0)
 
+// A buffer of a group and the bytes it needs.
+struct Part {
+  DevBuf* buf;
+  size_t bytes;
+};
+// Makes a group of buffers that grow together parts of one allocation: a context has
+// some fifty buffers, and what a small one spends on being made is allocations
+// (13 k tets: made in 3.9 ms, first 256x256 image 1.4; buffer by buffer 4.2 and 2.1.
+// 200 k tets with SH degree 3: made in 7.2 ms, first 800x800 image 2.2; 15.7 and 5.9).
+// When one of them is too small the whole group moves, none shrinks, and what they
+// held is gone (*grew).
+int ensure_group(RmeshCtx* c, DevBuf& block, std::initializer_list<Part> parts, bool* grew = nullptr) {
+  bool fits = true;
+  size_t total = 0;
+  auto want = [](const Part& q) { return (std::max(std::max<size_t>(q.bytes, 256), q.buf->bytes) + 255) / 256 * 256; };
+  for (const Part& q : parts) {
+    fits = fits && q.buf->p && q.bytes <= q.buf->bytes;
+    total += want(q);
+  }
+  if (fits) return RMESH_OK;
+  std::vector<size_t> sizes;
+  for (const Part& q : parts) {
+    sizes.push_back(want(q));
+    q.buf->release();
+  }
+  block.release();
+  CKR(ensure_buf(c, block, total));
+  char* at = block.as<char>();
+  size_t i = 0;
+  for (const Part& q : parts) {
+    q.buf->place(at, sizes[i]);
+    at += sizes[i++];
+  }
+  if (grew) *grew = true;
+  return RMESH_OK;
+}
+
 // ---------------------------------------------------------------- tile configurations
 // A tile configuration: tile size 8, 12 or 16 and the threads per tile (one per
 // pixel rounded up to whole warps, or twice that: WIDE).
@@ -380,10 +430,10 @@ struct ViewPlan {
 };
 
 // ---------------------------------------------------------------- sorting
-// hist: zeroed before the call
+// hist: zeroed before the call; status: sort_status_bytes(cap), zeroed when it was made
 template <typename K>
 int radix_sort(RmeshCtx* c, K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt, const void* n_ptr, int n_is_u64,
-               uint64_t cap, int bits, K** out_keys, uint32_t** out_vals, SortHist* hist) {
+               uint64_t cap, int bits, K** out_keys, uint32_t** out_vals, SortHist* hist, const DevBuf& status) {
   const int passes = std::max(1, (bits + 7) / 8);
   SortState* st = c->sort_state.as<SortState>();
   Counters* cnt = c->counters_d.as<Counters>();
@@ -399,7 +449,7 @@ int radix_sort(RmeshCtx* c, K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals
   uint32_t* vout = vals_alt;
   for (int p = 0; p < passes; ++p) {
     onesweep_kernel<K><<<grid, kSortThreads, smem, c->stream>>>(kin, vin, kout, vout, n_ptr, n_is_u64, cap, 8 * p, p,
-                                                                st, hist, c->sort_status.as<unsigned long long>(),
+                                                                st, hist, status.as<unsigned long long>(),
                                                                 &cnt->err);
     CKL();
     std::swap(kin, kout);
@@ -451,39 +501,38 @@ struct RunState {
   }
 };
 
-// Status words of a sort of up to n keys.  New memory is cleared: a word left there by
-// another context's sort of the same epoch would count as published.
-int ensure_sort_status(RmeshCtx* c, uint64_t n) {
-  const size_t had = c->sort_status.bytes;
-  CKR(ensure_buf(c, c->sort_status, ((n + kSortPart - 1) / kSortPart + 1) * 256 * 8));
-  if (c->sort_status.bytes != had) CK(cudaMemsetAsync(c->sort_status.p, 0, c->sort_status.bytes, c->stream));
-  return RMESH_OK;
-}
+// Status words of a sort of up to n keys.  New memory has to be cleared: a word left
+// there by another context's sort of the same epoch would count as published.
+size_t sort_status_bytes(uint64_t n) { return ((n + kSortPart - 1) / kSortPart + 1) * 256 * 8; }
 
 int ensure_run_buffers(RmeshCtx* c, int n_views, uint64_t total_pixels, uint32_t total_tiles) {
   const uint64_t items = (uint64_t)n_views * (uint64_t)c->M;
-  CKR(ensure_buf(c, c->vis_key, items * 8));
-  CKR(ensure_buf(c, c->vis_key_alt, items * 8));
-  CKR(ensure_buf(c, c->vis_val, items * 4));
-  CKR(ensure_buf(c, c->vis_val_alt, items * 4));
-  CKR(ensure_buf(c, c->vis_cnt, items * 4));
-  CKR(ensure_buf(c, c->group_off, ((items + 255) / 256 + 1) * 8));
-  CKR(ensure_buf(c, c->vis_proj, items * 32));
-  CKR(ensure_buf(c, c->vis_view, items * sizeof(TetView)));
-  if (c->sh_degree >= 0) {
-    CKR(ensure_buf(c, c->vis_color, items * 16));
-  }
+  CKR(ensure_group(c, c->item_mem,
+                   {{&c->vis_key, items * 8},
+                    {&c->vis_key_alt, items * 8},
+                    {&c->vis_val, items * 4},
+                    {&c->vis_val_alt, items * 4},
+                    {&c->vis_cnt, items * 4},
+                    {&c->group_off, ((items + 255) / 256 + 1) * 8},
+                    {&c->vis_proj, items * 32},
+                    {&c->vis_view, items * sizeof(TetView)},
+                    {&c->vis_color, c->sh_degree >= 0 ? items * 16 : 0}}));
   if (c->cap_pairs == 0) c->cap_pairs = std::min(std::max<uint64_t>(8 * items, 1u << 16), c->pair_limit);
-  CKR(ensure_buf(c, c->pair_key, c->cap_pairs * 4));
-  CKR(ensure_buf(c, c->pair_val, c->cap_pairs * 4));
-  CKR(ensure_buf(c, c->pair_key_alt, c->cap_pairs * 4));
-  CKR(ensure_buf(c, c->pair_val_alt, c->cap_pairs * 4));
-  CKR(ensure_buf(c, c->spans_fwd, c->cap_pairs * 4 * kSpanWords));
-  CKR(ensure_buf(c, c->spans_adj, c->cap_pairs * 4 * kSpanWords));
-  CKR(ensure_sort_status(c, std::max<uint64_t>(std::max<uint64_t>(items, c->cap_pairs), 4ull * c->M)));
-  CKR(ensure_buf(c, c->run_state, RunState(items, total_tiles).bytes));
-  CKR(ensure_buf(c, c->tile_order, (uint64_t)std::max<uint32_t>(total_tiles, 1) * 4));
-  CKR(ensure_buf(c, c->rgba, std::max<uint64_t>(total_pixels, 1) * 16));
+  bool grew = false;
+  CKR(ensure_group(c, c->pair_mem,
+                   {{&c->pair_key, c->cap_pairs * 4},
+                    {&c->pair_val, c->cap_pairs * 4},
+                    {&c->pair_key_alt, c->cap_pairs * 4},
+                    {&c->pair_val_alt, c->cap_pairs * 4},
+                    {&c->spans_fwd, c->cap_pairs * 4 * kSpanWords},
+                    {&c->spans_adj, c->cap_pairs * 4 * kSpanWords},
+                    {&c->sort_status, sort_status_bytes(std::max<uint64_t>(items, c->cap_pairs))}},
+                   &grew));
+  if (grew) CK(cudaMemsetAsync(c->sort_status.p, 0, c->sort_status.bytes, c->stream));
+  CKR(ensure_group(c, c->tile_mem,
+                   {{&c->run_state, RunState(items, total_tiles).bytes},
+                    {&c->tile_order, (uint64_t)std::max<uint32_t>(total_tiles, 1) * 4},
+                    {&c->rgba, std::max<uint64_t>(total_pixels, 1) * 16}}));
   return RMESH_OK;
 }
 
@@ -631,7 +680,7 @@ int run_bin(RmeshCtx* c, const ViewParams* views_dev, int n_views, uint32_t tota
     CKR(radix_sort<unsigned long long>(c, c->vis_key.as<unsigned long long>(), c->vis_val.as<uint32_t>(),
                                        c->vis_key_alt.as<unsigned long long>(), c->vis_val_alt.as<uint32_t>(),
                                        &cnt->n_vis, 0, items, 32, &tk, &tv,
-                                       reinterpret_cast<SortHist*>(state + rs.hist_a)));
+                                       reinterpret_cast<SortHist*>(state + rs.hist_a), c->sort_status));
   }
   {
     StageScope sc(c, kStEmit, capturing);
@@ -668,7 +717,7 @@ int run_bin(RmeshCtx* c, const ViewParams* views_dev, int n_views, uint32_t tota
     CKR(radix_sort<uint32_t>(c, c->pair_key.as<uint32_t>(), c->pair_val.as<uint32_t>(), c->pair_key_alt.as<uint32_t>(),
                              c->pair_val_alt.as<uint32_t>(), &cnt->n_pairs, 1, c->cap_pairs, bits,
                              &c->sorted_pair_key, &c->sorted_pair_val,
-                             reinterpret_cast<SortHist*>(state + rs.hist_b)));
+                             reinterpret_cast<SortHist*>(state + rs.hist_b), c->sort_status));
   }
   {
     StageScope sc(c, kStRanges, capturing);
@@ -1120,27 +1169,27 @@ int train_views(RmeshCtx* c, const RmeshCamera* cams, int n_views, const float* 
 
 int build_csr(RmeshCtx* c) {
   const uint64_t n_refs = 4ull * (uint64_t)c->M;
-  CKR(ensure_buf(c, c->csr_off, (c->N + 1) * 4));
-  CKR(ensure_buf(c, c->csr_ref, n_refs * 4));
-  DevBuf k0, k1, v1, nbuf, hist;
-  CKR(ensure_buf(c, k0, n_refs * 4));
-  CKR(ensure_buf(c, k1, n_refs * 4));
-  CKR(ensure_buf(c, v1, n_refs * 4));
-  CKR(ensure_buf(c, nbuf, 8));
-  CKR(ensure_buf(c, hist, sizeof(SortHist)));
+  DevBuf scratch, k0, k1, v1, nbuf, hist, status;  // (the allocation outlives its parts)
+  CKR(ensure_group(c, scratch,
+                   {{&k0, n_refs * 4},
+                    {&k1, n_refs * 4},
+                    {&v1, n_refs * 4},
+                    {&nbuf, 8},
+                    {&hist, sizeof(SortHist)},
+                    {&status, sort_status_bytes(n_refs)}}));
   CK(cudaMemsetAsync(hist.p, 0, sizeof(SortHist), c->stream));
+  CK(cudaMemsetAsync(status.p, 0, status.bytes, c->stream));
   const uint32_t n32 = (uint32_t)n_refs;
   CK(cudaMemcpyAsync(nbuf.p, &n32, 4, cudaMemcpyHostToDevice, c->stream));
   csr_fill_kernel<<<(unsigned)((n_refs + 255) / 256), 256, 0, c->stream>>>((int)c->M, c->idx.as<uint32_t>(),
                                                                           k0.as<uint32_t>(), c->csr_ref.as<uint32_t>());
   CKL();
-  CKR(ensure_sort_status(c, n_refs));
   CK(cudaMemsetAsync(c->counters_d.p, 0, sizeof(Counters), c->stream));
   uint32_t* ok_keys = nullptr;
   uint32_t* ok_vals = nullptr;
   CKR(radix_sort<uint32_t>(c, k0.as<uint32_t>(), c->csr_ref.as<uint32_t>(), k1.as<uint32_t>(), v1.as<uint32_t>(),
                            nbuf.p, 0, n_refs, std::max(1, bitlen((uint64_t)std::max<int64_t>(c->N - 1, 1))), &ok_keys,
-                           &ok_vals, hist.as<SortHist>()));
+                           &ok_vals, hist.as<SortHist>(), status));
   if (ok_vals != c->csr_ref.as<uint32_t>())
     CK(cudaMemcpyAsync(c->csr_ref.p, ok_vals, n_refs * 4, cudaMemcpyDeviceToDevice, c->stream));
   csr_offsets_kernel<<<(unsigned)((n_refs + 1 + 255) / 256), 256, 0, c->stream>>>((int)n_refs, (int)c->N, ok_keys,
@@ -1224,43 +1273,51 @@ int rmesh_create(const RmeshSceneDesc* d, RmeshCtx** out) {
   auto init = [&]() -> int {
     CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     c->own_stream = true;
-    CK(cudaMallocHost(&c->views_h, sizeof(ViewParams) * kMaxViews));
-    CK(cudaMallocHost(&c->counters_h, sizeof(Counters) * kMaxViews));
-    CK(cudaMallocHost(&c->hp_h, sizeof(AdamParams)));
+    {
+      constexpr size_t kViews = (sizeof(ViewParams) * kMaxViews + 255) / 256 * 256;
+      constexpr size_t kCounters = (sizeof(Counters) * kMaxViews + 255) / 256 * 256;
+      CK(cudaMallocHost(&c->host_mem, kViews + kCounters + sizeof(AdamParams)));
+      char* at = static_cast<char*>(c->host_mem);
+      c->views_h = reinterpret_cast<ViewParams*>(at);
+      c->counters_h = reinterpret_cast<Counters*>(at + kViews);
+      c->hp_h = reinterpret_cast<AdamParams*>(at + kViews + kCounters);
+    }
     const size_t N = (size_t)c->N, M = (size_t)c->M;
-    CKR(ensure_buf(c, c->verts, 3 * N * 4));
-    CKR(ensure_buf(c, c->idx, 4 * M * 4));
-    CKR(ensure_buf(c, c->dens, M * 4));
-    CKR(ensure_buf(c, c->cgrad, 3 * M * 4));
-    CKR(ensure_buf(c, c->base, 3 * M * 4));
-    CKR(ensure_buf(c, c->circ, 4 * M * 4));
-    DevBuf* zeros[] = {&c->m_verts, &c->v_verts, &c->m_dens, &c->v_dens, &c->m_cgrad, &c->v_cgrad, &c->m_base, &c->v_base};
-    size_t zsz[] = {3 * N, 3 * N, M, M, 3 * M, 3 * M, 3 * M, 3 * M};
-    for (int i = 0; i < 8; ++i) {
-      CKR(ensure_buf(c, *zeros[i], zsz[i] * 4));
-      CK(cudaMemsetAsync(zeros[i]->p, 0, zsz[i] * 4, c->stream));
+    const size_t n_sh = c->sh_degree >= 0 ? M * 3 * (size_t)c->sh_nc : 0, n_aux = M * (size_t)c->aux_dim;
+    CKR(ensure_group(c, c->scene_mem,
+                     {{&c->verts, 3 * N * 4},
+                      {&c->idx, 4 * M * 4},
+                      {&c->dens, M * 4},
+                      {&c->cgrad, 3 * M * 4},
+                      {&c->base, 3 * M * 4},
+                      {&c->circ, 4 * M * 4},
+                      {&c->sh, n_sh * 4},
+                      {&c->rec, M * sizeof(TetRec)},
+                      {&c->color4, M * 16},
+                      {&c->grad_slot, grad_floats(c) * 4},
+                      {&c->csr_off, (N + 1) * 4},
+                      {&c->csr_ref, 4 * M * 4},
+                      {&c->views_d, sizeof(ViewParams) * kMaxViews},
+                      {&c->counters_d, sizeof(Counters) * kMaxViews},
+                      {&c->hp_d, sizeof(AdamParams)},
+                      // zero at the start, from here to the end
+                      {&c->sort_state, sizeof(SortState)},
+                      {&c->m_verts, 3 * N * 4},
+                      {&c->v_verts, 3 * N * 4},
+                      {&c->m_dens, M * 4},
+                      {&c->v_dens, M * 4},
+                      {&c->m_cgrad, 3 * M * 4},
+                      {&c->v_cgrad, 3 * M * 4},
+                      {&c->m_base, 3 * M * 4},
+                      {&c->v_base, 3 * M * 4},
+                      {&c->m_sh, n_sh * 4},
+                      {&c->v_sh, n_sh * 4},
+                      {&c->aux_data, n_aux * 4}}));
+    {
+      char* from = c->sort_state.as<char>();
+      CK(cudaMemsetAsync(from, 0, c->scene_mem.as<char>() + c->scene_mem.bytes - from, c->stream));
     }
-    CKR(ensure_buf(c, c->rec, M * sizeof(TetRec)));
-    CKR(ensure_buf(c, c->color4, M * 16));
-    CKR(ensure_buf(c, c->grad_slot, grad_floats(c) * 4));
-    if (c->aux_dim > 0) {
-      CKR(ensure_buf(c, c->aux_data, M * (size_t)c->aux_dim * 4));
-      CK(cudaMemsetAsync(c->aux_data.p, 0, M * (size_t)c->aux_dim * 4, c->stream));
-    }
-    if (c->sh_degree >= 0) {
-      const size_t n_sh = M * 3 * (size_t)c->sh_nc;
-      CKR(ensure_buf(c, c->sh, n_sh * 4));
-      CKR(ensure_buf(c, c->m_sh, n_sh * 4));
-      CKR(ensure_buf(c, c->v_sh, n_sh * 4));
-      CK(cudaMemsetAsync(c->m_sh.p, 0, n_sh * 4, c->stream));
-      CK(cudaMemsetAsync(c->v_sh.p, 0, n_sh * 4, c->stream));
-      CKR(copy_in(c, c->sh, d->sh_coeffs, n_sh * 4));
-    }
-    CKR(ensure_buf(c, c->views_d, sizeof(ViewParams) * kMaxViews));
-    CKR(ensure_buf(c, c->counters_d, sizeof(Counters) * kMaxViews));
-    CKR(ensure_buf(c, c->hp_d, sizeof(AdamParams)));
-    CKR(ensure_buf(c, c->sort_state, sizeof(SortState)));
-    CK(cudaMemsetAsync(c->sort_state.p, 0, sizeof(SortState), c->stream));
+    if (n_sh) CKR(copy_in(c, c->sh, d->sh_coeffs, n_sh * 4));
     CKR(copy_in(c, c->verts, d->vertices, 3 * N * 4));
     CKR(copy_in(c, c->idx, d->indices, 4 * M * 4));
     {
@@ -1303,9 +1360,7 @@ int rmesh_destroy(RmeshCtx* c) {
   }
   for (auto e : c->event_pool) cudaEventDestroy(e);
   c->targets.close();
-  if (c->views_h) cudaFreeHost(c->views_h);
-  if (c->counters_h) cudaFreeHost(c->counters_h);
-  if (c->hp_h) cudaFreeHost(c->hp_h);
+  if (c->host_mem) cudaFreeHost(c->host_mem);
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
   delete c;
   return RMESH_OK;

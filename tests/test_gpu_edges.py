@@ -128,6 +128,29 @@ def test_contexts_that_inherit_memory(c1_scene, oracle32):
             r.close()
 
 
+def test_buffers_that_grow_in_any_order(c1_scene):
+    """One context takes views, view counts and pair counts up and down; buffers that
+    share an allocation move together.  Each image equals a fresh context's bit for bit,
+    each backward pass and step agrees to the order of its sums."""
+    from conftest import c1_camera
+
+    rng = np.random.default_rng(4)
+    one = make_renderer(c1_scene, c1_camera(64, 48))
+    for size, n in (((64, 48), 1), ((300, 200), 1), ((64, 48), 5), ((48, 64), 1), ((300, 200), 3), ((520, 410), 1)):
+        cam = c1_camera(*size)
+        new = make_renderer(c1_scene, cam)
+        for a, b in zip(one.forward_views([cam] * n), new.forward_views([cam] * n)):
+            np.testing.assert_array_equal(a, b)
+        gt = [rng.uniform(0, 1, (size[1], size[0], 3)).astype(np.float32) for _ in range(n)]
+        np.testing.assert_allclose(one.accumulate_views([cam] * n, gt, mode="graph"),
+                                   new.accumulate_views([cam] * n, gt, mode="graph"), rtol=1e-6)
+        m = 20 * one.n_tets
+        a, b = one.grad_slots().cpu().numpy()[:m], new.grad_slots().cpu().numpy()[:m]
+        assert rel_l2(a, b) <= 1e-5
+        new.close()
+    one.close()
+
+
 @pytest.mark.parametrize("where", ["host", "device"])
 def test_failing_forward_writes_nothing(c1_scene, where):
     """A view that needs more (tile, tet) slots than the context may hold fails; the
