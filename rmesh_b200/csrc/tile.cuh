@@ -215,14 +215,21 @@ __device__ __forceinline__ float rcp_fast(float x) {
   return r;
 }
 
+// num / den, correctly rounded, for 1e-20 <= |den| <= 2^60 and num 0 or 2^-60 <= |num|
+// <= 2^60, where no intermediate can overflow or lose bits: a Newton step makes y the
+// reciprocal to within rounding, and by Markstein's theorem (IBM J. Res. Dev. 34,
+// 1990) one fused residual step from q = num * y then rounds the quotient correctly.
+__device__ __forceinline__ float plain_quotient(float num, float den) {
+  float y = rcp_fast(den);
+  y = __fmaf_rn(y, __fmaf_rn(-den, y, 1.0f), y);
+  const float q = fm(num, y);
+  return __fmaf_rn(__fmaf_rn(-den, q, num), y, q);
+}
+
 // The same rules without branches, for planes whose numbers are in range (the
-// record's kPlainPlanes bit: no intermediate below can overflow or lose bits)
-// and a ray parallel to none of them; `plain` is false otherwise and the caller
-// takes intersect4.  The quotients are the correctly rounded ones: a Newton
-// step makes y the reciprocal to within rounding, and by Markstein's theorem
-// (IBM J. Res. Dev. 34, 1990) one fused residual step from q = num * y then
-// rounds num / den correctly.  FACES: also the faces that gave t_min (4: none)
-// and t_max.
+// record's kPlainPlanes bit) and a ray parallel to none of them; `plain` is false
+// otherwise and the caller takes intersect4.  FACES: also the faces that gave t_min
+// (4: none) and t_max.
 template <bool FACES>
 __device__ __forceinline__ bool intersect4_plain(const float4* nrm, float dx, float dy, float dz, float& t_min,
                                                  float& t_max, int& fmin, int& fmax, bool& plain) {
@@ -230,10 +237,7 @@ __device__ __forceinline__ bool intersect4_plain(const float4* nrm, float dx, fl
 #pragma unroll
   for (int f = 0; f < 4; ++f) {
     den[f] = dot3x(nrm[f].x, nrm[f].y, nrm[f].z, dx, dy, dz);
-    float y = rcp_fast(den[f]);
-    y = __fmaf_rn(y, __fmaf_rn(-den[f], y, 1.0f), y);
-    const float q0 = fm(nrm[f].w, y);
-    q[f] = __fmaf_rn(__fmaf_rn(-den[f], q0, nrm[f].w), y, q0);
+    q[f] = plain_quotient(nrm[f].w, den[f]);
   }
   plain = fminf(fminf(fabsf(den[0]), fabsf(den[1])), fminf(fabsf(den[2]), fabsf(den[3]))) >= 1e-20f;
   t_min = -3.402823e38f;
