@@ -789,23 +789,35 @@ int launch_tile_t(RmeshCtx* c, TileArgs& ta, uint32_t n_tiles, bool persistent) 
 
 // Rows per strip (4, 2 or 1) of a launch.  A strip is one warp's serial work, so
 // small launches take thinner strips until the chip has enough of them; thin strips
-// repeat the per-tet set-up more often and fill fewer pixel lanes.  Measured with
-// 12-pixel tiles (tile kernel, 4 / 2 / 1 rows, in units of 16 four-row strips per SM):
-//   forward + adjoint  2.3: 0.351 / 0.263 / 0.326 ms   2.5: 1.18 / 0.64 / 0.67 ms
-//                      4.3: 0.843 / 0.784 / 1.056 ms   9.4: 2.28 / 2.48 / 3.33 ms
-//                      79: 32.0 / 35.1 / 46.9 ms
-//   forward            0.6: 0.106 / 0.066 / 0.050 ms   8.1: 0.432 / 0.402 / 0.544 ms
-//                      45: 3.18 / 3.13 / 4.47 ms
-// The forward has little set-up and never gains from the four rows.  A wide
-// configuration (twice the threads per tile) takes two rows where the plain one takes
-// four; thinner than that it only lost (20,000 points at 1024x1024, one row instead of
-// two with 8- / 12-pixel tiles: forward call 1.70 / 1.38 against 1.15 / 0.96 ms, error
-// statistics 4.19 / 3.51 against 2.43 / 2.21; at 512x512 the fused step 1.43 / 1.27
-// against 0.96 / 0.93).
+// repeat the per-tet set-up more often and fill fewer pixel lanes.  Measured tile
+// kernel (ms, 4 / 2 / 1 rows), the launch's size in units of 16 four-row strips per SM:
+//   forward + adjoint
+//     8-pixel tiles   0.22: 0.785 / 0.514 / 0.355   0.86: 0.641 / 0.450 / 0.341
+//                     1.95: 0.574 / 0.416 / 0.660   3.46: 0.250 / 0.233 / 0.411 (13 k tets)
+//                     3.46: 0.573 / 0.617 / 1.086   4.14: 0.595 / 0.718   5.41: 0.731 / 0.908 / 1.625
+//                     13.8: 1.69 / 2.15 / 3.89      67.6: 9.05 / 11.7 / 21.4
+//     12-pixel tiles  0.15: 1.357 / 0.768 / 0.521   0.61: 1.055 / 0.607 / 0.381
+//                     1.30: 0.938 / 0.551 / 0.597   2.34: 0.912 / 0.566 / 0.957
+//                     3.69: 0.901 / 0.813 / 1.407   9.37: 1.89 / 1.87 / 3.27
+//                     45.5: 10.1 / 10.3 / 18.5      79: 32.0 / 35.1 / 46.9
+//     16-pixel tiles  0.43: 1.134 / 0.732 / 0.468   0.97: 1.141 / 0.622 / 0.558
+//                     1.73: 1.081 / 0.603 / 0.876   2.70: 1.024 / 0.832 / 1.283
+//                     6.92: 1.82 / 1.90 / 2.97      33.8: 9.82 / 10.5 / 16.8
+//   forward (2 / 1)
+//     8-pixel tiles   0.86: 0.164 / 0.111   1.95: 0.145 / 0.207
+//     12-pixel tiles  0.61: 0.205 / 0.130   1.30: 0.180 / 0.181   2.34: 0.187 / 0.285
+//     16-pixel tiles  0.97: 0.186 / 0.162   1.73: 0.182 / 0.251
+// (20,000 to 30,000 points unless said).  Four rows of an 8-pixel tile are 32 pixels,
+// one per lane, so they pay earlier than the 48 and 64 of the others.  The forward has
+// little set-up and never gains from the four rows.  A wide configuration (twice the
+// threads per tile) takes two rows where the plain one takes four; thinner than that it
+// only lost (20,000 points at 1024x1024, one row instead of two with 8- / 12-pixel
+// tiles: forward call 1.70 / 1.38 against 1.15 / 0.96 ms, error statistics 4.19 / 3.51
+// against 2.43 / 2.21; at 512x512 the fused step 1.43 / 1.27 against 0.96 / 0.93).
 int strip_rows(const RmeshCtx* c, uint32_t n_tiles, TileConf tc, bool adjoint) {
   const uint64_t strips4 = (uint64_t)n_tiles * (uint64_t)(tc.ts / 4);
-  const uint64_t warps = (uint64_t)c->num_sms * 16u;
-  const int rows = strips4 < warps ? 1 : (!adjoint || strips4 < 6 * warps ? 2 : 4);
+  const uint64_t unit = (uint64_t)c->num_sms * 16u;
+  const int rows = strips4 < unit ? 1 : (!adjoint || strips4 < (tc.ts == 8 ? 4 : 6) * unit ? 2 : 4);
   return tc.wide ? std::min(rows, 2) : rows;
 }
 

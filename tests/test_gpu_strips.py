@@ -65,15 +65,17 @@ def test_images_smaller_than_strips_and_remainders(c1_scene, oracle32, w, h, ts,
 
 def strip_view(ts, rows, fov=50.0):
     """A view, no multiple of the tile, whose adjoint takes ``rows`` rows per strip: one
-    below 16 four-row strips per SM, four from six times as many, two between."""
+    below 16 four-row strips per SM, four from six times as many (four times for 8-pixel
+    tiles), two between."""
     import torch
 
     from rmesh_b200.camera import make_camera
 
     unit = 16 * torch.cuda.get_device_properties(0).multi_processor_count
-    k = int(np.ceil(np.sqrt({1: 0.3, 2: 1.1, 4: 6.1}[rows] * unit / (ts // 4))))
+    four = 4 if ts == 8 else 6
+    k = int(np.ceil(np.sqrt({1: 0.3, 2: 1.1, 4: four}[rows] * unit / (ts // 4))))
     strips = k * k * (ts // 4)
-    assert rows == (1 if strips < unit else 2 if strips < 6 * unit else 4)
+    assert rows == (1 if strips < unit else 2 if strips < four * unit else 4)
     return make_camera((2.1, -1.9, 0.9), (0.0, 0.0, 0.0), fov, k * ts - 1, k * ts - 3)
 
 
