@@ -14,6 +14,7 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <initializer_list>
 #include <mutex>
@@ -117,9 +118,7 @@ struct RmeshCtx {
   int device = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
-  // allocations that the buffers below are parts of: the scene's, and the runs' by
-  // what their sizes follow (items, pairs, tiles and pixels)
-  DevBuf scene_mem, item_mem, pair_mem, tile_mem;
+  DevBuf scene_mem, run_mem;  // what the scene's and every run's buffers are parts of
   void* host_mem = nullptr;  // pinned: views_h, counters_h, hp_h
   SideCopy<CudaCopyApi> targets;  // host targets of a step, copied beside the binning
   int64_t N = 0, M = 0;
@@ -349,16 +348,18 @@ struct Part {
   DevBuf* buf;
   size_t bytes;
 };
+size_t part_bytes(size_t n) { return (std::max<size_t>(n, 256) + 255) / 256 * 256; }
 // Makes a group of buffers that grow together parts of one allocation: a context has
-// some fifty buffers, and what a small one spends on being made is allocations
-// (13 k tets: made in 3.9 ms, first 256x256 image 1.4; buffer by buffer 4.2 and 2.1.
-// 200 k tets with SH degree 3: made in 7.2 ms, first 800x800 image 2.2; 15.7 and 5.9).
+// some fifty buffers, and what a small one spends on being made is allocations, 0.33
+// ms each whatever the size unless the driver has room in memory that it mapped before.
+// (13 k tets: made in 3.3 ms, first 256x256 image 0.7; buffer by buffer 4.2 and 2.1.
+// 200 k tets with SH degree 3: made in 6.9 ms, first 800x800 image 1.6; 15.7 and 5.9).
 // When one of them is too small the whole group moves, none shrinks, and what they
 // held is gone (*grew).
 int ensure_group(RmeshCtx* c, DevBuf& block, std::initializer_list<Part> parts, bool* grew = nullptr) {
   bool fits = true;
   size_t total = 0;
-  auto want = [](const Part& q) { return (std::max(std::max<size_t>(q.bytes, 256), q.buf->bytes) + 255) / 256 * 256; };
+  auto want = [](const Part& q) { return part_bytes(std::max(q.bytes, q.buf->bytes)); };
   for (const Part& q : parts) {
     fits = fits && q.buf->p && q.bytes <= q.buf->bytes;
     total += want(q);
@@ -507,7 +508,9 @@ size_t sort_status_bytes(uint64_t n) { return ((n + kSortPart - 1) / kSortPart +
 
 int ensure_run_buffers(RmeshCtx* c, int n_views, uint64_t total_pixels, uint32_t total_tiles) {
   const uint64_t items = (uint64_t)n_views * (uint64_t)c->M;
-  CKR(ensure_group(c, c->item_mem,
+  if (c->cap_pairs == 0) c->cap_pairs = std::min(std::max<uint64_t>(8 * items, 1u << 16), c->pair_limit);
+  bool grew = false;
+  CKR(ensure_group(c, c->run_mem,
                    {{&c->vis_key, items * 8},
                     {&c->vis_key_alt, items * 8},
                     {&c->vis_val, items * 4},
@@ -516,23 +519,19 @@ int ensure_run_buffers(RmeshCtx* c, int n_views, uint64_t total_pixels, uint32_t
                     {&c->group_off, ((items + 255) / 256 + 1) * 8},
                     {&c->vis_proj, items * 32},
                     {&c->vis_view, items * sizeof(TetView)},
-                    {&c->vis_color, c->sh_degree >= 0 ? items * 16 : 0}}));
-  if (c->cap_pairs == 0) c->cap_pairs = std::min(std::max<uint64_t>(8 * items, 1u << 16), c->pair_limit);
-  bool grew = false;
-  CKR(ensure_group(c, c->pair_mem,
-                   {{&c->pair_key, c->cap_pairs * 4},
+                    {&c->vis_color, c->sh_degree >= 0 ? items * 16 : 0},
+                    {&c->pair_key, c->cap_pairs * 4},
                     {&c->pair_val, c->cap_pairs * 4},
                     {&c->pair_key_alt, c->cap_pairs * 4},
                     {&c->pair_val_alt, c->cap_pairs * 4},
                     {&c->spans_fwd, c->cap_pairs * 4 * kSpanWords},
                     {&c->spans_adj, c->cap_pairs * 4 * kSpanWords},
-                    {&c->sort_status, sort_status_bytes(std::max<uint64_t>(items, c->cap_pairs))}},
+                    {&c->sort_status, sort_status_bytes(std::max<uint64_t>(items, c->cap_pairs))},
+                    {&c->run_state, RunState(items, total_tiles).bytes},
+                    {&c->tile_order, (uint64_t)std::max<uint32_t>(total_tiles, 1) * 4},
+                    {&c->rgba, std::max<uint64_t>(total_pixels, 1) * 16}},
                    &grew));
   if (grew) CK(cudaMemsetAsync(c->sort_status.p, 0, c->sort_status.bytes, c->stream));
-  CKR(ensure_group(c, c->tile_mem,
-                   {{&c->run_state, RunState(items, total_tiles).bytes},
-                    {&c->tile_order, (uint64_t)std::max<uint32_t>(total_tiles, 1) * 4},
-                    {&c->rgba, std::max<uint64_t>(total_pixels, 1) * 16}}));
   return RMESH_OK;
 }
 
@@ -1179,17 +1178,30 @@ int train_views(RmeshCtx* c, const RmeshCamera* cams, int n_views, const float* 
   return fail(c, RMESH_ERR_PAIR_OVERFLOW, "pair buffers could not be grown enough");
 }
 
+std::array<Part, 6> csr_scratch(const RmeshCtx* c, DevBuf& k0, DevBuf& k1, DevBuf& v1, DevBuf& nbuf, DevBuf& hist,
+                                DevBuf& status) {
+  const size_t n_refs = 4 * (size_t)c->M;
+  return {Part{&k0, n_refs * 4}, Part{&k1, n_refs * 4},          Part{&v1, n_refs * 4},
+          Part{&nbuf, 8},        Part{&hist, sizeof(SortHist)}, Part{&status, sort_status_bytes(n_refs)}};
+}
+size_t csr_scratch_bytes(const RmeshCtx* c) {
+  DevBuf b;
+  size_t n = 0;
+  for (const Part& q : csr_scratch(c, b, b, b, b, b, b)) n += part_bytes(q.bytes);
+  return n;
+}
+
+// The vertex map: for each vertex the (tet, corner) references to it, ascending.
 int build_csr(RmeshCtx* c) {
   const uint64_t n_refs = 4ull * (uint64_t)c->M;
-  DevBuf scratch, k0, k1, v1, nbuf, hist, status;  // (the allocation outlives its parts)
-  CKR(ensure_group(c, scratch,
-                   {{&k0, n_refs * 4},
-                    {&k1, n_refs * 4},
-                    {&v1, n_refs * 4},
-                    {&nbuf, 8},
-                    {&hist, sizeof(SortHist)},
-                    {&status, sort_status_bytes(n_refs)}}));
-  CK(cudaMemsetAsync(hist.p, 0, sizeof(SortHist), c->stream));
+  // scratch in the gradient buffer, which no run has used yet
+  DevBuf k0, k1, v1, nbuf, hist, status;
+  char* at = c->grad_slot.as<char>();
+  for (const Part& q : csr_scratch(c, k0, k1, v1, nbuf, hist, status)) {
+    q.buf->place(at, q.bytes);
+    at += part_bytes(q.bytes);
+  }
+  CK(cudaMemsetAsync(hist.p, 0, hist.bytes, c->stream));
   CK(cudaMemsetAsync(status.p, 0, status.bytes, c->stream));
   const uint32_t n32 = (uint32_t)n_refs;
   CK(cudaMemcpyAsync(nbuf.p, &n32, 4, cudaMemcpyHostToDevice, c->stream));
@@ -1306,7 +1318,7 @@ int rmesh_create(const RmeshSceneDesc* d, RmeshCtx** out) {
                       {&c->sh, n_sh * 4},
                       {&c->rec, M * sizeof(TetRec)},
                       {&c->color4, M * 16},
-                      {&c->grad_slot, grad_floats(c) * 4},
+                      {&c->grad_slot, std::max(grad_floats(c) * 4, csr_scratch_bytes(c))},
                       {&c->csr_off, (N + 1) * 4},
                       {&c->csr_ref, 4 * M * 4},
                       {&c->views_d, sizeof(ViewParams) * kMaxViews},
@@ -1350,6 +1362,7 @@ int rmesh_create(const RmeshSceneDesc* d, RmeshCtx** out) {
     CKR(copy_in(c, c->base, d->base_colors, 3 * M * 4));
     CKR(copy_in(c, c->circ, d->circumdata, 4 * M * 4));
     CKR(build_csr(c));
+    CK(cudaMemsetAsync(c->grad_slot.p, 0, c->grad_slot.bytes, c->stream));  // no gradients yet
     return RMESH_OK;
   };
   r = init();
