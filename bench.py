@@ -52,19 +52,26 @@ LR_SH = 2.5e-3
 # (smsp__inst_executed.sum), each from a one-pass ncu capture of this workload's
 # step (--profile-one-step --tile-size T: 38.33 M pairs at 12, 8.30 GB and 35.07 G;
 # 58.17 M pairs at 8, 7.93 GB and 31.71 G).  The issue ceiling is 148 SMs x 4
-# schedulers x one instruction per clock.  Sizes without a capture report null.
+# schedulers x one instruction per clock.  They hold for that step only: other tile
+# sizes, meshes and views report null.
 TILE_DRAM_BYTES_PER_PAIR = {12: 216.6, 8: 136.4}
 TILE_WARP_INST_PER_PAIR = {12: 915.0, 8: 545.0}
 
 
-def dram_traffic(n_pairs: int, tile_size: int):
-    per_pair = TILE_DRAM_BYTES_PER_PAIR.get(tile_size)
+def per_pair_count(table, args, tile_size: int):
+    counted = (args.workload == "batched" and args.points == 100_000 and args.views == N_VIEWS
+               and tuple(args.res) == RES and args.sh_degree == 3)
+    return table.get(tile_size) if counted else None
+
+
+def dram_traffic(n_pairs: int, args, tile_size: int):
+    per_pair = per_pair_count(TILE_DRAM_BYTES_PER_PAIR, args, tile_size)
     return None if per_pair is None else int(per_pair * n_pairs)
 
 
-def issue_roofline(n_pairs: int, launch_ms: float, sm_mhz, tile_size: int):
+def issue_roofline(n_pairs: int, launch_ms: float, sm_mhz, args, tile_size: int):
     """The tile kernel's bound in practice: instruction issue, not HBM."""
-    per_pair = TILE_WARP_INST_PER_PAIR.get(tile_size)
+    per_pair = per_pair_count(TILE_WARP_INST_PER_PAIR, args, tile_size)
     if per_pair is None:
         return None
     mhz = float(sm_mhz) if sm_mhz else 1965.0
@@ -337,13 +344,13 @@ def run_gpu(args):
         "stage_ms_per_step": {k: round(v / nsteps_prof, 4) for k, v in stage_ms.items()},
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 4),
-                     "traffic": dram_traffic(int(info.n_pairs_last), tile_size),
+                     "traffic": dram_traffic(int(info.n_pairs_last), args, tile_size),
                      "kernel": f"strip_kernel<{tile_size},kModeTrain> (fused forward+loss+adjoint, "
                                f"one warp per strip of tile rows)",
                      "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else
                      "fallback 6.65 TB/s", "launch_ms": round(comp_ms, 4), "algorithmic_bytes": alg,
                      "n_pairs": int(info.n_pairs_last)},
-        "issue_roofline": issue_roofline(int(info.n_pairs_last), comp_ms, clocks.get("sm_mhz"), tile_size),
+        "issue_roofline": issue_roofline(int(info.n_pairs_last), comp_ms, clocks.get("sm_mhz"), args, tile_size),
         "clocks": clocks,
     }
     if rank == 0 and not args.no_cpu_baseline:
@@ -631,13 +638,13 @@ def run_training(args):
         "stage_ms_per_step": {k: round(v / nb, 4) for k, v in stage_ms.items()},
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 4),
-                     "traffic": dram_traffic(int(info.n_pairs_last), tile[0]),
+                     "traffic": dram_traffic(int(info.n_pairs_last), args, tile[0]),
                      "kernel": f"strip_kernel<{tile[0]},kModeTrain> (fused forward+loss+adjoint, "
                                f"one warp per strip of tile rows)",
                      "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else
                      "fallback 6.65 TB/s", "launch_ms": round(comp_ms, 4), "algorithmic_bytes": alg,
                      "n_pairs": int(info.n_pairs_last)},
-        "issue_roofline": issue_roofline(int(info.n_pairs_last), comp_ms, clocks.get("sm_mhz"), tile[0]),
+        "issue_roofline": issue_roofline(int(info.n_pairs_last), comp_ms, clocks.get("sm_mhz"), args, tile[0]),
         "clocks": clocks,
         "training": {"lr_verts": lr["lr_verts"],
                      "loss_first_pass": fin(losses[:nb].mean()), "loss_last_pass": fin(losses[-nb:].mean()),

@@ -33,3 +33,24 @@ def test_reference_arm_json_line():
     # the line states the work it timed: its sampled steps fit in the run's wall time
     assert d["steps"] * d["ms_per_step"] / 1e3 <= wall
     assert d["full_step_ms_estimate"] > 0
+
+
+def test_counted_figures_only_for_the_counted_step():
+    """DRAM bytes and instructions per pair were counted on the default step; a larger
+    mesh has other pairs, and its line must not scale them (its issue rate would read
+    above the hardware's)."""
+    import argparse
+
+    import bench
+
+    def args(**kw):
+        d = dict(workload="batched", points=100_000, views=16, res=bench.RES, sh_degree=3)
+        return argparse.Namespace(**{**d, **kw})
+
+    assert bench.dram_traffic(1000, args(), 8) == 136_400
+    assert bench.issue_roofline(53_161_336, 33.33, 1965.0, args(), 8)["frac"] < 1.0
+    for other in (args(points=1_000_000), args(workload="large"), args(views=8), args(res=((64, 64),)),
+                  args(sh_degree=-1)):
+        assert bench.dram_traffic(1000, other, 8) is None
+        assert bench.issue_roofline(1000, 1.0, 1965.0, other, 8) is None
+    assert bench.dram_traffic(1000, args(), 16) is None
