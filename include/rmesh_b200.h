@@ -175,8 +175,9 @@ RMESH_API int rmesh_forward_tiled(RmeshCtx* ctx, const RmeshCamera* cam, float* 
  * rmesh_train_step_views): n_views cameras of any sizes rendered by one
  * persistent launch.  rgba_out receives the views' [H][W][4] images back to
  * back, aux_out (optional) their [H][W][8 + aux_dim] aux images back to back.
- * Images equal rmesh_forward_tiled's per view; a failing run writes nothing.  rmesh_backward does not
- * follow this call (it follows a single-view rmesh_forward_tiled). */
+ * Images equal rmesh_forward_tiled's per view; a failing run writes nothing.
+ * rmesh_backward does not follow this call (it follows a single-view
+ * rmesh_forward_tiled). */
 RMESH_API int rmesh_forward_views(RmeshCtx* ctx, const RmeshCamera* cams, int32_t n_views, float* rgba_out,
                                   float* aux_out);
 
@@ -356,10 +357,11 @@ RMESH_API int rmesh_debug_ranges(RmeshCtx* ctx, uint32_t* ranges, uint64_t n_til
  * 2^31 - 1), so that a run which needs more fails with RMESH_ERR_PAIR_OVERFLOW. */
 RMESH_API int rmesh_debug_limit_pairs(RmeshCtx* ctx, uint64_t limit);
 
-/* No reference counterpart: runs the path's two bounded waits (chained-scan
- * look-back, TMA mbarrier) on conditions that never resolve and returns, in
- * bits_out[0..1], the error bits each wait recorded after giving up (2 =
- * RMESH spin timeout).  The device stays usable; used by the failure tests. */
+/* No reference counterpart: runs two bounded waits (the path's chained-scan
+ * look-back, and an mbarrier's, which no kernel of the path uses) on conditions
+ * that never resolve and returns, in bits_out[0..1], the error bits each wait
+ * recorded after giving up (2 = RMESH spin timeout).  The device stays usable;
+ * used by the failure tests. */
 RMESH_API int rmesh_debug_timeouts(uint32_t* bits_out);
 
 /* ---- profiling -------------------------------------------------------------- */

@@ -1228,10 +1228,10 @@ int build_csr(RmeshCtx* c) {
 
 }  // namespace
 
-// Exercises the two bounded waits of the path on conditions that never
-// resolve: a chained-scan look-back whose predecessor never publishes
-// (status[0] stays 0) and an mbarrier phase that never completes.  Each wait
-// gives up after its limit and records kErrSpinTimeout in bits[0] / bits[1];
+// Exercises two bounded waits on conditions that never resolve: the path's
+// chained-scan look-back with a predecessor that never publishes (status[0] stays
+// 0), and an mbarrier phase that never completes (no kernel of the path waits on
+// one; the ABI's probe reports both).  Each wait gives up after its limit and records kErrSpinTimeout in bits[0] / bits[1];
 // the kernel then returns normally.
 __global__ void timeout_probe_kernel(unsigned long long* status, uint32_t* bits) {
   __shared__ uint64_t bar;

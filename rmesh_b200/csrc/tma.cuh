@@ -1,6 +1,6 @@
-// Asynchronous copies into shared memory, and the bounded mbarrier wait (sm_90+
-// PTX, used on sm_100a).  Every copy reads this GPU's own memory, 16 bytes at
-// 16-byte aligned addresses.
+// Asynchronous copies into shared memory (every copy reads this GPU's own memory,
+// 16 bytes at 16-byte aligned addresses), and the bounded mbarrier wait of the
+// timeout probe (sm_90+ PTX, used on sm_100a).
 #pragma once
 #include <stdint.h>
 

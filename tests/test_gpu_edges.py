@@ -2,8 +2,8 @@
 nothing, a camera inside the mesh (negative depth keys, vertices behind the
 camera), a multi-view step whose tiles exceed 2^16 in total, pair-buffer
 overflow, tile lists of thousands of tets, the reference's grid mesh,
-its cross-renderer cameras, and tets large enough that a batch's covered
-pixels exceed the kernel's sub-batch capacity."""
+its cross-renderer cameras, tets that cover more than a tile, calls that
+fail, contexts that inherit memory and buffers that grow in any order."""
 from __future__ import annotations
 
 import numpy as np
@@ -200,8 +200,7 @@ def test_failing_forward_writes_nothing(c1_scene, where):
 
 def test_long_tile_lists(c2_scene):
     """65k tets seen at 48x48 (16 tiles of 12x12): each tile's list holds
-    thousands of tets (hundreds of 32-tet batches, each with its span records
-    bulk-copied beside its tet records, the forward stopping at the
+    thousands of tets (hundreds of 32-tet batches, the forward stopping at the
     transmittance cut-off long before the adjoint's end of the list); losses
     and parameters of the persistent batched path equal the plain path's."""
     from rmesh_b200.camera import orbit_cameras
@@ -322,12 +321,9 @@ def _max_batch_items(sc, cam, ref, ts):
 @pytest.mark.parametrize("ts", [8, 12, 16])
 def test_large_tets_many_sub_batches(oracle32, ts):
     """60 points -> 287 tets, most covering more than a tile at 128x96: a
-    tile's 32-tet batch then holds more covered pixels than the kernel's
-    per-sub-batch item capacity (512; 800 for 12-pixel tiles), so batches
-    split into sub-batches, whose item maps are written in the previous
-    sub-batch's tail.  Forward image, tile
-    lists, adjoint gradients, error statistics and a batched / graph-mode
-    training step against the oracle."""
+    tile's 32-tet batch covers up to 953, 1,660 and 2,497 pixels at tiles of 8,
+    12 and 16.  Forward image, tile lists, adjoint gradients, error statistics
+    and a batched / graph-mode training step against the oracle."""
     from oracle import OracleTrainer
     from rmesh_b200.camera import make_camera
     from rmesh_b200.scenes import make_scene, uniform_cloud
@@ -340,8 +336,7 @@ def test_large_tets_many_sub_batches(oracle32, ts):
     r = make_renderer(sc, cam, tile_size=ts)
     img = r.forward_tiled(cam.cam_pos, cam.vp, cam.c2w_intrinsics)
     ref = oracle32.forward_tiled(sc, cam, tile_size=ts)
-    # some batches exceed the kernel's sub-batch capacity (953, 1,660 and 2,497
-    # items at tiles of 8, 12 and 16)
+    # batches of 953, 1,660 and 2,497 items at tiles of 8, 12 and 16
     assert _max_batch_items(sc, cam, ref, ts) > (800 if ts == 12 else 512)
     tiles, tets = r.debug_pairs()
     np.testing.assert_array_equal(tiles, ref["key_hi"])
